@@ -54,12 +54,30 @@ struct FastDiv {
 __host__ __device__ __forceinline__ float2 mul_i(float2 a) { return make_float2(-a.y, a.x); }
 __host__ __device__ __forceinline__ float2 mul_mi(float2 a) { return make_float2(a.y, -a.x); }
 
-// exp(i*phi) with the argument reduced in double precision first, then evaluated in float.
+// exp(i*phi): the argument is reduced to the nearest quarter turn in double precision and the
+// remainder, |r| <= pi/4, goes through the Taylor polynomials of sine and cosine (to r^9 and
+// r^10: truncation below 2e-9).  Rounding the remainder rather than an angle of up to pi to
+// float keeps the phase to 3e-8 (an angle near pi carries 1.2e-7), and nothing branches.
 __device__ __forceinline__ float2 expi_reduced(double phi) {
-  double r = phi - kTwoPi * rint(phi * kInvTwoPi);
-  float s, c;
-  sincosf((float)r, &s, &c);
-  return make_float2(c, s);
+  const double t = phi * (4.0 * kInvTwoPi);
+  const double q = rint(t);
+  const float r = (float)((t - q) * (0.25 * kTwoPi));
+  const float r2 = r * r;
+  const float ps = fmaf(r2, fmaf(r2, fmaf(r2, (float)(1.0 / 362880.0), (float)(-1.0 / 5040.0)),
+                                 (float)(1.0 / 120.0)), (float)(-1.0 / 6.0));
+  const float pc = fmaf(r2, fmaf(r2, fmaf(r2, fmaf(r2, (float)(-1.0 / 3628800.0),
+                                                   (float)(1.0 / 40320.0)),
+                                          (float)(-1.0 / 720.0)), (float)(1.0 / 24.0)), -0.5f);
+  const float s = fmaf(r * r2, ps, r), c = fmaf(r2, pc, 1.0f);
+  const int k = (int)(long long)q;
+  const float cx = (k & 1) ? s : c, sx = (k & 1) ? c : s;
+  return make_float2(((k + 1) & 2) ? -cx : cx, (k & 2) ? -sx : sx);
+}
+
+// a * (hi + lo), a scale held as the sum of two floats: 1/N in one float would give every
+// element of every pass the same relative error, up to 6e-8, and twenty passes add them up.
+__device__ __forceinline__ float2 cscale2(float2 a, float hi, float lo) {
+  return make_float2(fmaf(a.x, hi, a.x * lo), fmaf(a.y, hi, a.y * lo));
 }
 
 // Ampere-style asynchronous global -> shared copies (16 bytes; both addresses 16-byte aligned).
@@ -215,10 +233,11 @@ enum WaitFault : unsigned {
   WF_SELFTEST = 0x100u,
 };
 
-// Allow `bytes` of dynamic shared memory for `kernel` (only needed above the 48 KB default).
+// Allow `bytes` of dynamic shared memory for `kernel` (needed where it and the kernel's static
+// shared memory, at most 16 KB, pass the 48 KB default).
 template <typename K>
 inline cudaError_t allow_smem(K kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
+  if (bytes <= 32 * 1024) return cudaSuccess;
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 

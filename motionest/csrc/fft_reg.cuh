@@ -135,6 +135,20 @@ template <bool INV> struct RDft<9, INV> : RDftComp<3, 3, INV> {};
 template <bool INV> struct RDft<12, INV> : RDftComp<4, 3, INV> {};
 template <bool INV> struct RDft<14, INV> : RDftComp<2, 7, INV> {};
 template <bool INV> struct RDft<16, INV> : RDftComp<4, 4, INV> {};
+// radices of the run-time plans only (fft_rt.cuh)
+template <bool INV> struct RDft<10, INV> : RDftComp<2, 5, INV> {};
+template <bool INV> struct RDft<15, INV> : RDftComp<3, 5, INV> {};
+template <bool INV> struct RDft<18, INV> : RDftComp<2, 9, INV> {};
+template <bool INV> struct RDft<20, INV> : RDftComp<4, 5, INV> {};
+template <bool INV> struct RDft<21, INV> : RDftComp<3, 7, INV> {};
+template <bool INV> struct RDft<22, INV> : RDftComp<2, 11, INV> {};
+template <bool INV> struct RDft<24, INV> : RDftComp<4, 6, INV> {};
+template <bool INV> struct RDft<25, INV> : RDftComp<5, 5, INV> {};
+template <bool INV> struct RDft<26, INV> : RDftComp<2, 13, INV> {};
+template <bool INV> struct RDft<27, INV> : RDftComp<3, 9, INV> {};
+template <bool INV> struct RDft<28, INV> : RDftComp<4, 7, INV> {};
+template <bool INV> struct RDft<30, INV> : RDftComp<5, 6, INV> {};
+template <bool INV> struct RDft<32, INV> : RDftComp<4, 8, INV> {};
 
 // Second-stage twiddle W_N^{r j} from the plan-ordered table: for each r the R1 threads of a
 // line read R1 consecutive entries (one L1 wavefront per warp instead of one sector per

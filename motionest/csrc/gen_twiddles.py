@@ -21,7 +21,8 @@ PLANS = {
     88: (8, 11), 96: (16, 6), 112: (16, 7), 128: (16, 8), 144: (16, 9), 176: (16, 11),
     192: (16, 12), 224: (16, 14), 256: (16, 16),
 }
-RADICES = [2, 3, 4, 5, 6, 7, 8, 9, 11, 12, 13, 14, 16]
+RADICES = [2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 18, 20, 21, 22, 24, 25, 26, 27,
+           28, 30, 32]
 
 
 def f32(v):

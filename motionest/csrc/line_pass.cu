@@ -11,6 +11,7 @@
 
 #include "fft_reg.cuh"
 #include "line_pass.cuh"
+#include "phase.cuh"
 
 namespace me {
 
@@ -38,46 +39,6 @@ static bool fast_passes_enabled() {
 #ifndef ME_DUAL_SINGLE_BUFFER
 #define ME_DUAL_SINGLE_BUFFER 1
 #endif
-
-struct PhaseCoef {
-  double a, b, dm;
-};
-
-__device__ __forceinline__ PhaseCoef phase_coef(const Phase& P, const double* prm, int ax) {
-  PhaseCoef c{0.0, 0.0, 0.0};
-  if (P.kind != PH_NONE) {
-    const double th = prm[3 + P.rot];
-    if (P.kind == PH_TAN) {
-      const double t = tan(th * 0.5);
-      c.a = t;
-      c.dm = 0.5 * (1.0 + t * t);
-    } else {
-      c.a = -sin(th);
-      c.dm = -cos(th);
-    }
-  }
-  if (P.trans) c.b = -prm[ax];
-  return c;
-}
-
-__device__ __forceinline__ bool phase_is_identity(const Phase& P) {
-  return P.kind == PH_NONE && !P.trans && !P.trans_deriv && !P.deriv;
-}
-
-// Phase factor for frequency index n along the pass axis at spatial coordinates c[0..2]
-// (c[ax] is ignored by the planes, which are constant or broadcast along the pass axis in
-// frequency; c[ax] carries n itself).
-__device__ __forceinline__ float2 phase_value(const Phase& P, const PhaseCoef& C, int n,
-                                              const int c[3], float scale) {
-  double rk = 0.0, kn = 0.0;
-  if (P.plane) rk = P.plane[c[0] * P.ps[0] + c[1] * P.ps[1] + c[2] * P.ps[2]];
-  if (P.kv) kn = P.kv[n];
-  float2 e = expi_reduced(C.a * rk + C.b * kn);
-  if (P.deriv) e = cscale(mul_i(e), (float)(C.dm * rk));
-  if (P.trans_deriv) e = cscale(mul_mi(e), (float)kn);
-  if (P.conj) e = cconj(e);
-  return cscale(e, scale);
-}
 
 // Global element offset of (line l, index n) inside a volume.
 __device__ __forceinline__ i64 elem_offset(const PassArgs& A, int l, int n) {
@@ -183,13 +144,13 @@ __global__ void __launch_bounds__(256) line_pass_kernel(const PassArgs A) {
     int c[3];
     line_coords(A, l0 + min(b, max(nl - 1, 0)), n, c);
     const float2 v0 = R[n * A.es + b];
-    const float2 f0 = id0 ? make_float2(A.scale, 0.f) : phase_value(A.ph[0], c0, n, c, A.scale);
+    const float2 f0 = id0 ? make_float2(A.scale, 0.f) : phase_value(A.ph[0], c0, n, c, A.scale, A.scale_lo);
     if (MODE == PM_DUAL_OUT) {
-      const float2 f1 = id1 ? make_float2(A.scale, 0.f) : phase_value(A.ph[1], c1, n, c, A.scale);
+      const float2 f1 = id1 ? make_float2(A.scale, 0.f) : phase_value(A.ph[1], c1, n, c, A.scale, A.scale_lo);
       R[n * A.es + b] = cmul(v0, f0);
       R[n * A.es + B + b] = cmul(v0, f1);
     } else if (MODE == PM_DUAL_IN) {
-      const float2 f1 = id1 ? make_float2(A.scale, 0.f) : phase_value(A.ph[1], c1, n, c, A.scale);
+      const float2 f1 = id1 ? make_float2(A.scale, 0.f) : phase_value(A.ph[1], c1, n, c, A.scale, A.scale_lo);
       const float2 v1 = R[n * A.es + B + b];
       R[n * A.es + b] = cadd(cmul(v0, f0), cmul(v1, f1));
     } else {
@@ -231,11 +192,11 @@ struct LineChirp {
   // a line: even lanes evaluate the plain step, odd lanes the wrapping one, and the line's
   // first two lanes hand them to the rest (every lane of the warp must call init).
   __device__ __forceinline__ void init(const Phase& P, const PhaseCoef& Cf, double r_o, int j,
-                                       float scale, int G) {
+                                       float scale, float scale_lo, int G) {
     const double d = kTwoPi / N;
     const double C = (P.conj ? -1.0 : 1.0) * (Cf.a * r_o + Cf.b) * d;
     m = ((j - N / 2) % N + N) % N;
-    e = cscale(expi_reduced(C * ((double)m - 0.5 * N)), scale);
+    e = cscale2(expi_reduced(C * ((double)m - 0.5 * N)), scale, scale_lo);
     const float2 sv = expi_reduced(C * ((j & 1) ? (double)(R1 - N) : (double)R1));
     const int lead = (threadIdx.x & 31) & ~(G - 1);
     step = make_float2(__shfl_sync(0xffffffffu, sv.x, lead), __shfl_sync(0xffffffffu, sv.y, lead));
@@ -382,35 +343,35 @@ __global__ void __launch_bounds__(256, ME_PASS_MINB) fast_pass_kernel(const Pass
     const bool sep1 = kDual && !id1 && A.ph[1].sep;
     const PhaseCoef c0 = coef_s[0];
     const PhaseCoef c1 = kDual ? coef_s[1] : PhaseCoef{0, 0, 0};
-    if (sep0) ch0.init(A.ph[0], c0, A.ph[0].rvec ? A.ph[0].rvec[c[A.ph[0].oaxis]] : 0.0, j, A.scale, G);
-    if (sep1) ch1.init(A.ph[1], c1, A.ph[1].rvec ? A.ph[1].rvec[c[A.ph[1].oaxis]] : 0.0, j, A.scale, G);
+    if (sep0) ch0.init(A.ph[0], c0, A.ph[0].rvec ? A.ph[0].rvec[c[A.ph[0].oaxis]] : 0.0, j, A.scale, A.scale_lo, G);
+    if (sep1) ch1.init(A.ph[1], c1, A.ph[1].rvec ? A.ph[1].rvec[c[A.ph[1].oaxis]] : 0.0, j, A.scale, A.scale_lo, G);
     // V (element n = j + r R1 in slot r) times the factors of phase 0 or 1; which form applies
     // (identity, line chirp, per-element evaluation) is decided once per line
     auto factor0 = [&](float2 (&V)[R2]) {
       if (id0) {
 #pragma unroll
-        for (int r = 0; r < R2; r++) V[r] = cscale(V[r], A.scale);
+        for (int r = 0; r < R2; r++) V[r] = cscale2(V[r], A.scale, A.scale_lo);
       } else if (sep0) {
         ch0.apply(V);
       } else {
 #pragma unroll
         for (int r = 0; r < R2; r++) {
           c[A.ax] = j + r * R1;
-          V[r] = cmul(V[r], phase_value(A.ph[0], c0, j + r * R1, c, A.scale));
+          V[r] = cmul(V[r], phase_value(A.ph[0], c0, j + r * R1, c, A.scale, A.scale_lo));
         }
       }
     };
     auto factor1 = [&](float2 (&V)[R2]) {
       if (id1) {
 #pragma unroll
-        for (int r = 0; r < R2; r++) V[r] = cscale(V[r], A.scale);
+        for (int r = 0; r < R2; r++) V[r] = cscale2(V[r], A.scale, A.scale_lo);
       } else if (sep1) {
         ch1.apply(V);
       } else {
 #pragma unroll
         for (int r = 0; r < R2; r++) {
           c[A.ax] = j + r * R1;
-          V[r] = cmul(V[r], phase_value(A.ph[1], c1, j + r * R1, c, A.scale));
+          V[r] = cmul(V[r], phase_value(A.ph[1], c1, j + r * R1, c, A.scale, A.scale_lo));
         }
       }
     };
@@ -617,33 +578,33 @@ __global__ void __launch_bounds__(256, ME_PASS_MINB)
     const bool sep1 = kDual && !id1 && A.ph[1].sep;
     const PhaseCoef c0 = coef_s[0];
     const PhaseCoef c1 = kDual ? coef_s[1] : PhaseCoef{0, 0, 0};
-    if (sep0) ch0.init(A.ph[0], c0, A.ph[0].rvec ? A.ph[0].rvec[c[A.ph[0].oaxis]] : 0.0, j, A.scale, G);
-    if (sep1) ch1.init(A.ph[1], c1, A.ph[1].rvec ? A.ph[1].rvec[c[A.ph[1].oaxis]] : 0.0, j, A.scale, G);
+    if (sep0) ch0.init(A.ph[0], c0, A.ph[0].rvec ? A.ph[0].rvec[c[A.ph[0].oaxis]] : 0.0, j, A.scale, A.scale_lo, G);
+    if (sep1) ch1.init(A.ph[1], c1, A.ph[1].rvec ? A.ph[1].rvec[c[A.ph[1].oaxis]] : 0.0, j, A.scale, A.scale_lo, G);
     auto factor0 = [&](float2 (&V)[R2]) {
       if (id0) {
 #pragma unroll
-        for (int r = 0; r < R2; r++) V[r] = cscale(V[r], A.scale);
+        for (int r = 0; r < R2; r++) V[r] = cscale2(V[r], A.scale, A.scale_lo);
       } else if (sep0) {
         ch0.apply(V);
       } else {
 #pragma unroll
         for (int r = 0; r < R2; r++) {
           c[A.ax] = j + r * R1;
-          V[r] = cmul(V[r], phase_value(A.ph[0], c0, j + r * R1, c, A.scale));
+          V[r] = cmul(V[r], phase_value(A.ph[0], c0, j + r * R1, c, A.scale, A.scale_lo));
         }
       }
     };
     auto factor1 = [&](float2 (&V)[R2]) {
       if (id1) {
 #pragma unroll
-        for (int r = 0; r < R2; r++) V[r] = cscale(V[r], A.scale);
+        for (int r = 0; r < R2; r++) V[r] = cscale2(V[r], A.scale, A.scale_lo);
       } else if (sep1) {
         ch1.apply(V);
       } else {
 #pragma unroll
         for (int r = 0; r < R2; r++) {
           c[A.ax] = j + r * R1;
-          V[r] = cmul(V[r], phase_value(A.ph[1], c1, j + r * R1, c, A.scale));
+          V[r] = cmul(V[r], phase_value(A.ph[1], c1, j + r * R1, c, A.scale, A.scale_lo));
         }
       }
     };
@@ -949,15 +910,11 @@ int make_pass_args(int mode, const float2* in0, const float2* in1, float2* out0,
   A.pstride = pstride;
   A.ph[0] = f0;
   A.ph[1] = f1;
-  switch (mode) {
-    case PM_SHEAR:
-    case PM_DUAL_OUT:
-    case PM_DUAL_IN:
-      A.scale = 1.0f / (float)N;
-      break;
-    default:
-      A.scale = (float)(1.0 / sqrt((double)N));
-  }
+  const double gain = N * (fast_passes_enabled() ? fft_pair_gain(N) : 1.0);
+  const bool pair = mode == PM_SHEAR || mode == PM_DUAL_OUT || mode == PM_DUAL_IN;
+  const double scale = pair ? 1.0 / gain : 1.0 / sqrt(gain);
+  A.scale = (float)scale;
+  A.scale_lo = (float)(scale - (double)A.scale);
   *out = A;
   return ME_OK;
 }
@@ -974,7 +931,8 @@ int launch_line_pass(int mode, const float2* in0, const float2* in1, float2* out
   if (rc0 != ME_OK) return rc0;
   if (A.nlines == 0) return ME_OK;
   if (fast_passes_enabled()) {
-    const int rc = try_fast(mode, A, stream);
+    int rc = try_fast(mode, A, stream);
+    if (rc < 0) rc = try_rt_pass(mode, A, stream);
     if (rc >= 0) return rc;
   }
   switch (mode) {
@@ -1097,21 +1055,21 @@ __global__ void __launch_bounds__(256, ME_PASS_MINB)
     const bool sep0 = !id0 && A.ph[0].sep;
     const PhaseCoef c0 = coef_s;
     Ch ch0;
-    if (sep0) ch0.init(A.ph[0], c0, A.ph[0].rvec ? A.ph[0].rvec[c[A.ph[0].oaxis]] : 0.0, j, A.scale, G);
+    if (sep0) ch0.init(A.ph[0], c0, A.ph[0].rvec ? A.ph[0].rvec[c[A.ph[0].oaxis]] : 0.0, j, A.scale, A.scale_lo, G);
     float2* L0 = buf + g * LS;
     float2 X[R2];
     F::forward(L0, j, X);
     if (j < R1) {
       if (id0) {
 #pragma unroll
-        for (int r = 0; r < R2; r++) X[r] = cscale(X[r], A.scale);
+        for (int r = 0; r < R2; r++) X[r] = cscale2(X[r], A.scale, A.scale_lo);
       } else if (sep0) {
         ch0.apply(X);
       } else {
 #pragma unroll
         for (int r = 0; r < R2; r++) {
           c[A.ax] = j + r * R1;
-          X[r] = cmul(X[r], phase_value(A.ph[0], c0, j + r * R1, c, A.scale));
+          X[r] = cmul(X[r], phase_value(A.ph[0], c0, j + r * R1, c, A.scale, A.scale_lo));
         }
       }
     }
@@ -1246,7 +1204,7 @@ __global__ void __launch_bounds__(256, ME_PASS_MINB)
     const bool sep0 = !id0 && A.ph[0].sep;
     const PhaseCoef c0 = coef_s;
     Ch ch0;
-    if (sep0) ch0.init(A.ph[0], c0, A.ph[0].rvec ? A.ph[0].rvec[c[A.ph[0].oaxis]] : 0.0, j, A.scale, G);
+    if (sep0) ch0.init(A.ph[0], c0, A.ph[0].rvec ? A.ph[0].rvec[c[A.ph[0].oaxis]] : 0.0, j, A.scale, A.scale_lo, G);
     unsigned char* tb = tiles + cur * TILE;
     float2* L = scratch + g * LS;
     float2 X[R2];
@@ -1255,14 +1213,14 @@ __global__ void __launch_bounds__(256, ME_PASS_MINB)
     if (j < R1) {
       if (id0) {
 #pragma unroll
-        for (int r = 0; r < R2; r++) X[r] = cscale(X[r], A.scale);
+        for (int r = 0; r < R2; r++) X[r] = cscale2(X[r], A.scale, A.scale_lo);
       } else if (sep0) {
         ch0.apply(X);
       } else {
 #pragma unroll
         for (int r = 0; r < R2; r++) {
           c[A.ax] = j + r * R1;
-          X[r] = cmul(X[r], phase_value(A.ph[0], c0, j + r * R1, c, A.scale));
+          X[r] = cmul(X[r], phase_value(A.ph[0], c0, j + r * R1, c, A.scale, A.scale_lo));
         }
       }
     }

@@ -55,7 +55,7 @@ struct PassArgs {
   int B;   // lines per CTA
   int es;  // shared-memory row stride (elements)
   int accum;
-  float scale;
+  float scale, scale_lo;  // the pass's scale and what its rounding to float left
   const double* params;
   int pstride;
   Phase ph[2];
@@ -78,6 +78,14 @@ int make_pass_args(int mode, const float2* in0, const float2* in1, float2* out0,
 // lengths with compile-time FFTs) in one persistent launch.
 constexpr int kMaxMultiJobs = 16;
 int launch_multi_shear(const PassArgs* jobs, int njobs, cudaStream_t stream);
+
+// Mean gain of a forward and inverse FFT of length n with the float twiddles of its plan
+// (1 - 1e-8 .. 1 - 4e-8, the same for every element and pass, so that twenty passes would add it
+// up); scales divide by it.  1 for a length without a two-stage plan.
+double fft_pair_gain(int n);
+
+// The pass on the run-time two-stage FFT (rt_pass.cu); -1 when its length has no such plan.
+int try_rt_pass(int mode, PassArgs& A, cudaStream_t stream);
 
 // Launch one pass.  Returns ME_OK or an error code (error message set).
 int launch_line_pass(int mode, const float2* in0, const float2* in1, float2* out0, float2* out1,

@@ -22,6 +22,7 @@
 #include "fft_reg.cuh"
 #include "line_pass.cuh"
 #include "rigid.cuh"
+#include "sense.cuh"
 
 namespace me {
 
@@ -31,56 +32,10 @@ namespace me {
     if (_rc != ME_OK) return _rc; \
   } while (0)
 
-enum FwdMode { FWD_K = 0, FWD_RESID = 1, FWD_LM = 2 };
-
 // Resident CTAs per SM the fast SENSE kernels are compiled for (register budget 65536/(256*n)).
 #ifndef ME_SENSE_MINB
 #define ME_SENSE_MINB 2
 #endif
-constexpr int kLmStats = 28;  // e0, g[6], H upper triangle[21]
-constexpr int kThreads = 256;
-
-__host__ __device__ inline int pad2(int n) { return (n + 1) & ~1; }
-
-struct FwdArgs {
-  int X, Y, Z, C;
-  const float2* mps;
-  const float2* vols;
-  i64 vol_stride;
-  int shot0;
-  const int* shot_off;
-  const int* kx;
-  const int* ky;
-  const float2* ydat;
-  float2* kout;  // offsets relative to shot_off[shot0], or absolute when kout_abs
-  int kout_abs;
-  int vps;       // volumes per shot (compile-time kernels, V = 1): vols holds [shot][vps] volumes
-  i64 kout_vs;   // distance between the K regions of a shot's volumes
-  double* partial;
-  int XR, es;
-  float scale;
-  int bulk;  // stage rows with bulk copies (bases 16-byte aligned; set on the host)
-  FftPlan plan;
-};
-
-template <int NV>
-__device__ __forceinline__ void block_reduce_store(double (&v)[NV], double* out) {
-  __shared__ double red[kThreads / 32][NV > 1 ? NV : 1];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < NV; k++) {
-    double a = v[k];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-    if (lane == 0) red[warp][k] = a;
-  }
-  __syncthreads();
-  if (threadIdx.x < NV) {
-    double a = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) a += red[w][threadIdx.x];
-    out[threadIdx.x] = a;
-  }
-}
 
 // Gauss-Newton sums of one sample: |r|^2, Re(conj(r) J_p) and Re(conj(J_p) J_q) for q >= p.
 __device__ __forceinline__ void lm_accumulate(double (&st)[kLmStats], float2 r, const float2 (&J)[6]) {
@@ -207,24 +162,6 @@ __global__ void __launch_bounds__(kThreads) sense_fwd_kernel(const FwdArgs A) {
   }
 }
 
-struct AdjArgs {
-  int X, Y, Z, C;
-  const float2* mps;
-  const float2* kin;
-  int kin_rel;  // kin offsets relative to shot_off[shot0] (K workspace) or absolute (ydat)
-  float2* out;
-  i64 vol_stride;
-  int shot0;
-  const int* shot_off;
-  const int* kx;
-  const int* ky_off;
-  const int* ky_order;  // may be null
-  int XB, es;
-  float scale;
-  int bulk;  // stage map rows with bulk copies (bases 16-byte aligned; set on the host)
-  FftPlan plan;
-};
-
 template <int EPT>
 __global__ void __launch_bounds__(kThreads) sense_adj_kernel(const AdjArgs A) {
   extern __shared__ float2 sm[];
@@ -306,16 +243,6 @@ __device__ __forceinline__ void init_twiddles_any(float2* tw, int n) {
   } else {
     init_twiddles(tw, n);
   }
-}
-
-// (a * b) mod n for 0 <= a, b < n <= 512 (product < 2^18: exact in float).
-__device__ __forceinline__ int mulmod(int a, int b, int n, float inv_n) {
-  const int p = a * b;
-  int q = __float2int_rd((float)p * inv_n);
-  int r = p - q * n;
-  if (r < 0) r += n;
-  if (r >= n) r -= n;
-  return r;
 }
 
 // Rows per chunk of the forward kernel (one row per thread group) and its shared-memory plan.
@@ -1109,6 +1036,20 @@ static me_layout zxy_layout(const me_sense* pb) {
 
 static i64 vox_of(const me_sense* pb) { return (i64)pb->nx * pb->ny * pb->nz; }
 
+static bool fast_sense_enabled() {
+  static int v = -1;
+  if (v < 0) {
+    const char* e = getenv("ME_GENERIC_FFT");
+    v = (e && e[0] == '1') ? 0 : 1;
+  }
+  return v == 1;
+}
+
+// 1/sqrt(XY), with the gain of the FFT along y taken out
+static double sense_scale(const me_sense* pb) {
+  return 1.0 / sqrt((double)pb->nx * pb->ny * (fast_sense_enabled() ? fft_pair_gain(pb->ny) : 1.0));
+}
+
 static int fwd_rows(int V, int Y) {
   int xr = (V == 1) ? 16 : 4;
   while (xr > 1 && 2 * (i64)Y * (V * xr + 1) * 8 > 160 * 1024) xr /= 2;
@@ -1154,15 +1095,6 @@ static bool fused_lm_enabled() {
   static int v = -1;
   if (v < 0) {
     const char* e = getenv("ME_LM_TWO_PASS");
-    v = (e && e[0] == '1') ? 0 : 1;
-  }
-  return v == 1;
-}
-
-static bool fast_sense_enabled() {
-  static int v = -1;
-  if (v < 0) {
-    const char* e = getenv("ME_GENERIC_FFT");
     v = (e && e[0] == '1') ? 0 : 1;
   }
   return v == 1;
@@ -1271,10 +1203,11 @@ static bool has_fast_length(int n) {
   }
 }
 
-// Whether the compile-time SENSE kernels serve this problem (they take the K of several
-// volumes per shot in one launch, which the LM statistics use).
+// Whether the compile-time or run-time SENSE kernels serve this problem (they take the K of
+// several volumes per shot in one launch, which the LM statistics use).
 static bool fast_sense_for(const me_sense* pb) {
-  return fast_sense_enabled() && pb->nx <= 512 && has_fast_length(pb->ny);
+  return fast_sense_enabled() && pb->nx <= 512 &&
+         (has_fast_length(pb->ny) || has_rt_sense(pb->ny));
 }
 
 static int launch_fwd(const me_sense* pb, int mode, const float2* vols, i64 vol_stride, int shot0,
@@ -1298,7 +1231,9 @@ static int launch_fwd(const me_sense* pb, int mode, const float2* vols, i64 vol_
   A.ydat = (const float2*)pb->ydat;
   A.kout = kout;
   A.partial = partial;
-  A.scale = (float)(1.0 / sqrt((double)pb->nx * pb->ny));
+  const double scale = sense_scale(pb);
+  A.scale = (float)scale;
+  A.scale_lo = (float)(scale - (double)A.scale);
   if (!make_plan(pb->ny, &A.plan)) {
     set_error("ny has a prime factor > 13");
     return ME_ERR_UNSUPPORTED;
@@ -1310,11 +1245,12 @@ static int launch_fwd(const me_sense* pb, int mode, const float2* vols, i64 vol_
     // FWD_LM over the seven volumes of each shot: the fused statistics kernel, or -1 (not
     // handled) for the caller's two-kernel path
     if (mode == FWD_LM && vps == 7) return fused_lm_enabled() ? try_fast_lm(A, maxps, nb, st) : -1;
-    const int rc = try_fast_fwd(A, mode, maxps, nb, st);
+    int rc = try_fast_fwd(A, mode, maxps, nb, st);
+    if (rc < 0) rc = try_rt_fwd(A, mode, maxps, nb, st);
     if (rc >= 0) return rc;
   }
   if (vps != 1) {
-    set_error("several volumes per shot need the compile-time SENSE kernels");
+    set_error("several volumes per shot need the compile-time or run-time SENSE kernels");
     return ME_ERR_UNSUPPORTED;
   }
   if (mode == FWD_LM) {
@@ -1360,14 +1296,17 @@ static int launch_adj(const me_sense* pb, const float2* kin, int kin_rel, float2
   A.kx = pb->samples.kx;
   A.ky_off = pb->samples.ky_off;
   A.ky_order = pb->samples.ky_order;
-  A.scale = (float)(1.0 / sqrt((double)pb->nx * pb->ny));
+  const double scale = sense_scale(pb);
+  A.scale = (float)scale;
+  A.scale_lo = (float)(scale - (double)A.scale);
   if (!make_plan(pb->ny, &A.plan)) {
     set_error("ny has a prime factor > 13");
     return ME_ERR_UNSUPPORTED;
   }
   A.bulk = bulk_enabled() && al16(A.mps) && pb->ny % 2 == 0;
   if (fast_sense_enabled() && pb->nx <= 512) {
-    const int rc = try_fast_adj(A, pb->samples.max_per_shot, nb, st);
+    int rc = try_fast_adj(A, pb->samples.max_per_shot, nb, st);
+    if (rc < 0) rc = try_rt_adj(A, pb->samples.max_per_shot, nb, st);
     if (rc >= 0) return rc;
   }
   A.XB = std::max(1, std::min(std::min(pb->nx, 32), 4096 / pb->ny));

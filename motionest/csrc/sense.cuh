@@ -1,0 +1,88 @@
+// Arguments and helpers shared by the SENSE kernels (sense.cu, rt_sense.cu).
+#pragma once
+#include "fft_smem.cuh"
+
+namespace me {
+
+enum FwdMode { FWD_K = 0, FWD_RESID = 1, FWD_LM = 2 };
+
+constexpr int kLmStats = 28;  // e0, g[6], H upper triangle[21]
+constexpr int kThreads = 256;
+
+__host__ __device__ inline int pad2(int n) { return (n + 1) & ~1; }
+
+struct FwdArgs {
+  int X, Y, Z, C;
+  const float2* mps;
+  const float2* vols;
+  i64 vol_stride;
+  int shot0;
+  const int* shot_off;
+  const int* kx;
+  const int* ky;
+  const float2* ydat;
+  float2* kout;  // offsets relative to shot_off[shot0], or absolute when kout_abs
+  int kout_abs;
+  int vps;       // volumes per shot (compile-time kernels, V = 1): vols holds [shot][vps] volumes
+  i64 kout_vs;   // distance between the K regions of a shot's volumes
+  double* partial;
+  int XR, es;
+  float scale, scale_lo;  // 1/sqrt(XY) and what its rounding to float left
+  int bulk;  // stage rows with bulk copies (bases 16-byte aligned; set on the host)
+  FftPlan plan;
+};
+
+template <int NV>
+__device__ __forceinline__ void block_reduce_store(double (&v)[NV], double* out) {
+  __shared__ double red[kThreads / 32][NV > 1 ? NV : 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < NV; k++) {
+    double a = v[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+    if (lane == 0) red[warp][k] = a;
+  }
+  __syncthreads();
+  if (threadIdx.x < NV) {
+    double a = 0.0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); w++) a += red[w][threadIdx.x];
+    out[threadIdx.x] = a;
+  }
+}
+
+struct AdjArgs {
+  int X, Y, Z, C;
+  const float2* mps;
+  const float2* kin;
+  int kin_rel;  // kin offsets relative to shot_off[shot0] (K workspace) or absolute (ydat)
+  float2* out;
+  i64 vol_stride;
+  int shot0;
+  const int* shot_off;
+  const int* kx;
+  const int* ky_off;
+  const int* ky_order;  // may be null
+  int XB, es;
+  float scale, scale_lo;
+  int bulk;  // stage map rows with bulk copies (bases 16-byte aligned; set on the host)
+  FftPlan plan;
+};
+
+// (a * b) mod n for 0 <= a, b < n <= 512 (product < 2^18: exact in float).
+__device__ __forceinline__ int mulmod(int a, int b, int n, float inv_n) {
+  const int p = a * b;
+  int q = __float2int_rd((float)p * inv_n);
+  int r = p - q * n;
+  if (r < 0) r += n;
+  if (r >= n) r -= n;
+  return r;
+}
+
+// The kernels on the run-time two-stage FFT (rt_sense.cu); -1 when ny has no such plan or the
+// mode is not theirs (FWD_LM).
+int try_rt_fwd(FwdArgs& A, int mode, int maxps, int nb, cudaStream_t st);
+int try_rt_adj(AdjArgs& A, int maxps, int nb, cudaStream_t st);
+bool has_rt_sense(int ny);
+
+}  // namespace me
