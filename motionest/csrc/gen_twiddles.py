@@ -55,6 +55,14 @@ def main():
         vals = ", ".join(f"{{{f32(np.cos(a))}, {f32(np.sin(a))}}}" for a in ang)
         lines.append(f"__device__ const float2 twp{n}[{r1 * r2}] = {{{vals}}};")
     lines.append("")
+    lines.append("// The twiddles of the line passes' plans N = G R1, G = 8 up to 128 points, else 16")
+    lines.append("// (pass_line.cuh): tp_<N>[r R1 + k] = exp(-2 pi i r k / N), r < G, k < R1.")
+    for n in sorted(PLANS):
+        g = 8 if n <= 128 else 16
+        ang = [-2.0 * np.pi * (r * k) / n for r in range(g) for k in range(n // g)]
+        vals = ", ".join(f"{{{f32(np.cos(a))}, {f32(np.sin(a))}}}" for a in ang)
+        lines.append(f"__device__ const float2 tp_{n}[{n}] = {{{vals}}};")
+    lines.append("")
     lines.append("// cos / sin of 2 pi m / R for the register DFTs (m is a compile-time constant at")
     lines.append("// every call site after unrolling, so these fold to immediates)")
     lines.append("template <int R> struct RadixConst;")

@@ -6,12 +6,11 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 
-#include "fft_reg.cuh"
-#include "line_pass.cuh"
-#include "phase.cuh"
+#include "pass_line.cuh"
 
 namespace me {
 
@@ -27,18 +26,6 @@ static bool fast_passes_enabled() {
   }
   return v == 1;
 }
-
-// Resident CTAs per SM the compile-time pass kernels are compiled for.
-#ifndef ME_PASS_MINB
-#define ME_PASS_MINB 2
-#endif
-// 1: the two-line-set (dual) modes keep one tile buffer instead of two, so that two CTAs fit
-// on an SM (the next tile is then loaded after the current one is stored, not during it, and
-// the other CTA's work covers the load).  Measured on the LM statistics at 256x224x176:
-// 696 ms against 712 ms with two buffers and one CTA per SM.
-#ifndef ME_DUAL_SINGLE_BUFFER
-#define ME_DUAL_SINGLE_BUFFER 1
-#endif
 
 // Global element offset of (line l, index n) inside a volume.
 __device__ __forceinline__ i64 elem_offset(const PassArgs& A, int l, int n) {
@@ -173,143 +160,88 @@ __global__ void __launch_bounds__(256) line_pass_kernel(const PassArgs A) {
 }
 
 // ------------------------------------------------------------------ compile-time lengths
-// Same contract as line_pass_kernel, with the line FFT in registers (fft_reg.cuh): one group
-// of G threads per line, B = 256 / G lines per tile, no CTA-wide barrier between FFT stages.
-// CTAs are persistent over (volume, tile) work items and prefetch the next tile with
-// asynchronous copies into a second buffer while the current one is transformed.
+// The pass for the compile-time lengths (pass_line.cuh): tiles of 16 lines, eight or sixteen
+// threads a line, CTAs that are persistent over (volume, tile) work items and load the next tile
+// while the current one is transformed.  The dual modes keep one buffer of two tiles (the
+// next tile is then loaded after the current one is stored, and the other CTAs of the SM cover
+// the load).
+//
+// What bounds it: instruction issue (DFTs, chirp, slot accesses) and, from 200 points on, DRAM.
+// CTAs per SM it is compiled for: 16 warps of 128 registers, 20 of 96 at the shortest lengths.
+constexpr int pass_min_ctas(int n, bool dual) { return n > 128 ? 2 : (dual || n > 64) ? 4 : 5; }
 
-// Chirp of one line by recurrence along its elements n = j + r*R1 (r < R2):
-// f = mult(n) * exp(i C (m(n) - N/2)), m(n) = (n - N/2) mod N, C = (a r_o + b) 2 pi / N.
-template <int N, int R1, int R2>
-struct LineChirp {
-  float2 e, step, stepw;  // current factor (output scale folded in), step by R1, step with wrap
-  int m;
-  float dmr;   // deriv multiplier per unit (m - N/2): dm * r_o * 2 pi / N
-  float tdr;   // translation-derivative multiplier per unit: 2 pi / N
-  bool deriv, tderiv, conj;
-  // A conjugated phase is conjugated once here: conj(e s^r) = conj(e) conj(s)^r, and the
-  // i / -i of the derivative multipliers swap.  The two steps are the same for the G lanes of
-  // a line: even lanes evaluate the plain step, odd lanes the wrapping one, and the line's
-  // first two lanes hand them to the rest (every lane of the warp must call init).
-  __device__ __forceinline__ void init(const Phase& P, const PhaseCoef& Cf, double r_o, int j,
-                                       float scale, float scale_lo, int G) {
-    const double d = kTwoPi / N;
-    const double C = (P.conj ? -1.0 : 1.0) * (Cf.a * r_o + Cf.b) * d;
-    m = ((j - N / 2) % N + N) % N;
-    e = cscale2(expi_reduced(C * ((double)m - 0.5 * N)), scale, scale_lo);
-    const float2 sv = expi_reduced(C * ((j & 1) ? (double)(R1 - N) : (double)R1));
-    const int lead = (threadIdx.x & 31) & ~(G - 1);
-    step = make_float2(__shfl_sync(0xffffffffu, sv.x, lead), __shfl_sync(0xffffffffu, sv.y, lead));
-    stepw = make_float2(__shfl_sync(0xffffffffu, sv.x, lead + 1),
-                        __shfl_sync(0xffffffffu, sv.y, lead + 1));
-    dmr = (float)(Cf.dm * r_o * d);
-    tdr = (float)d;
-    deriv = P.deriv != 0;
-    tderiv = P.trans_deriv != 0;
-    conj = P.conj != 0;
-  }
-  __device__ __forceinline__ float2 value() const {
-    float2 f = e;
-    const float mm = (float)m - 0.5f * N;
-    if (deriv) f = cscale(conj ? mul_mi(f) : mul_i(f), dmr * mm);
-    if (tderiv) f = cscale(conj ? mul_i(f) : mul_mi(f), tdr * mm);
-    return f;
-  }
-  __device__ __forceinline__ void advance() {
-    m += R1;
-    if (m >= N) {
-      m -= N;
-      e = cmul(e, stepw);
-    } else {
-      e = cmul(e, step);
-    }
-  }
-  // V[r] *= f(j + r R1) for the thread's R2 elements, with the branch on the multiplier taken
-  // once for the line rather than per element
-  __device__ __forceinline__ void apply(float2 (&V)[R2]) {
-    if (deriv || tderiv) {
-#pragma unroll
-      for (int r = 0; r < R2; r++) {
-        V[r] = cmul(V[r], value());
-        advance();
-      }
-    } else {
-#pragma unroll
-      for (int r = 0; r < R2; r++) {
-        V[r] = cmul(V[r], e);
-        advance();
-      }
-    }
-  }
-};
+// Bytes between the lines of a linear tile: 16-byte multiples, 64 modulo 128.
+constexpr int line_pitch(int n) { return n * 8 + (n % 16 == 0 ? 64 : 0); }
 
-template <int N, int R1, int R2, int MODE>
-__global__ void __launch_bounds__(256, ME_PASS_MINB) fast_pass_kernel(const PassArgs A) {
-  using F = LineFft<N, R1, R2>;
-  using Ch = LineChirp<N, R1, R2>;
-  constexpr int G = F::G;
-  constexpr int B = 256 / G;
-  constexpr int LS = F::LS;
+// Coefficients of volume `vol`'s phases into shared memory when the CTA moves to another volume
+// (uniform over the CTA, so the barrier is too); their last readers are past a barrier.
+template <bool kDual>
+__device__ __forceinline__ void set_coefs(const PassArgs& A, int vol, int& coef_vol,
+                                          PhaseCoef* coef_s) {
+  if (vol == coef_vol) return;
+  if (threadIdx.x < (kDual ? 2 : 1)) {
+    PhaseCoef cf{0, 0, 0};
+    if (A.params) cf = phase_coef(A.ph[threadIdx.x], A.params + (i64)vol * A.pstride, A.ax);
+    coef_s[threadIdx.x] = cf;
+  }
+  coef_vol = vol;
+  __syncthreads();
+}
+
+// Tile staging by cp.async: any strides and alignments, and the plain FFT modes.
+template <int N, int MODE>
+__global__ void __launch_bounds__(PassLine<N>::THREADS,
+                                  pass_min_ctas(N, MODE == PM_DUAL_IN || MODE == PM_DUAL_OUT))
+    fast_pass_kernel(const __grid_constant__ PassArgs A) {
+  constexpr int G = PassLine<N>::G, B = kTileLines;
   constexpr bool kDual = (MODE == PM_DUAL_IN || MODE == PM_DUAL_OUT);
-  constexpr int NREG = kDual ? 2 * B : B;
-  constexpr int NBUF = (kDual && ME_DUAL_SINGLE_BUFFER) ? 1 : 2;  // tile buffers
-  extern __shared__ __align__(16) float2 smem[];
+  constexpr int NT = kDual ? 2 : 1;    // tiles per buffer
+  constexpr int NBUF = kDual ? 1 : 2;
+  constexpr int PITCH = line_pitch(N), TILE = B * PITCH;
+  extern __shared__ __align__(128) unsigned char tiles[];
   __shared__ i64 lb_s[2][B];  // line base offsets of the tile in each buffer
+  __shared__ PhaseCoef coef_s[2];
 
   const int tiles_per_vol = (A.nlines + B - 1) / B;
   const int total = tiles_per_vol * A.nvol;
   const i64 sa = A.st[A.ax];
   const bool bfast = (A.st[A.av] == 1);
   const int dv = A.dims[A.av];
-  const int g = threadIdx.x / G;
-  const int j = threadIdx.x % G;
-  const bool id0 = phase_is_identity(A.ph[0]);
-  const bool id1 = phase_is_identity(A.ph[1]);
+  int g, j;
+  line_place<G>(g, j);
+  __shared__ float2 chirp_s[kTileLines][2 * G];
+  // this thread's line and first index when it copies: over the lines where they are neighbours
+  // in memory, else along its own line
+  const int cb = bfast ? threadIdx.x % B : threadIdx.x / G;
+  const int cn = bfast ? threadIdx.x / B : threadIdx.x % G;
+  Slots<G, false> s0, s1;
+  s0.init(g, j);
+  s1 = s0;
 
   auto line_base = [&](int l) {
     const int u = A.div_av.div(l);
     return (i64)u * A.st[A.au] + (i64)(l - u * dv) * A.st[A.av];
   };
-  // issue the loads of work item t into buffer `bufi`; line offsets computed once per line
-  // (the caller has synchronised, so lb_s[bufi] is free)
+  // issue the loads of work item t into buffer `bufi` (the caller has synchronised)
   auto issue = [&](int t, int bufi) {
     const int vol = A.div_tiles.div(t);
     const int l0 = (t - vol * tiles_per_vol) * B;
     const int nl = min(B, A.nlines - l0);
-    float2* buf = smem + bufi * NREG * LS;
     if (threadIdx.x < B) lb_s[bufi][threadIdx.x] = line_base(l0 + min((int)threadIdx.x, nl - 1));
-    // each thread computes the offsets of the lines it copies itself (no barrier needed)
-    const int nsrc = (MODE == PM_DUAL_IN) ? 2 : 1;
-    for (int k = 0; k < nsrc; k++) {
-      const float2* src = (k == 0 ? A.in0 : A.in1) + (i64)vol * A.in_vs;
-      if (bfast) {
-        // b = e % B is fixed per thread (256 is a multiple of B)
-        const int b = threadIdx.x % B;
-        const i64 base = line_base(l0 + min(b, nl - 1));
-        float2* dst0 = buf + (k * B + b) * LS;
-        for (int n = threadIdx.x / B; n < N; n += 256 / B) {
-          if (b < nl) cp_async8(dst0 + n, src + base + n * sa);
-          else dst0[n] = make_float2(0.f, 0.f);
-        }
-      } else {
-        // contiguous lines: one line per group of G = 256 / B threads, n fastest
-        const int b = threadIdx.x / G;
-        const i64 base = line_base(l0 + min(b, nl - 1));
-        float2* dst0 = buf + (k * B + b) * LS;
-        for (int n = threadIdx.x % G; n < N; n += G) {
-          if (b < nl) cp_async8(dst0 + n, src + base + n * sa);
-          else dst0[n] = make_float2(0.f, 0.f);
-        }
+    const i64 base = line_base(l0 + min(cb, nl - 1));
+#pragma unroll
+    for (int k = 0; k < (MODE == PM_DUAL_IN ? 2 : 1); k++) {
+      const float2* src = (k == 0 ? A.in0 : A.in1) + (i64)vol * A.in_vs + base;
+      float2* dst = reinterpret_cast<float2*>(tiles + (bufi * NT + k) * TILE + cb * PITCH);
+      for (int n = cn; n < N; n += G) {
+        if (cb < nl) cp_async8(dst + n, src + n * sa);
+        else dst[n] = make_float2(0.f, 0.f);
       }
     }
     cp_async_commit();
   };
 
-  int cur = 0;
-  // The shear coefficients depend on the volume only: one thread sets them up in shared memory
-  // when the CTA moves to another volume (vol is uniform over the CTA, so the barrier is too).
-  __shared__ PhaseCoef coef_s[2];
-  int coef_vol = -1;
+  int cur = 0, coef_vol = -1;
   if ((int)blockIdx.x < total) issue(blockIdx.x, 0);
   for (int t = blockIdx.x; t < total; t += gridDim.x) {
     const int vol = A.div_tiles.div(t);
@@ -318,128 +250,23 @@ __global__ void __launch_bounds__(256, ME_PASS_MINB) fast_pass_kernel(const Pass
     cp_async_wait_all();
     __syncthreads();
     if (NBUF == 2 && t + (int)gridDim.x < total) issue(t + gridDim.x, cur ^ 1);
-    float2* buf = smem + cur * NREG * LS;
-
-    // per-line phase set-up
-    if (vol != coef_vol) {
-      if (threadIdx.x < (kDual ? 2 : 1)) {
-        PhaseCoef cf{0, 0, 0};
-        if (A.params) cf = phase_coef(A.ph[threadIdx.x], A.params + (i64)vol * A.pstride, A.ax);
-        coef_s[threadIdx.x] = cf;
-      }
-      coef_vol = vol;
-      __syncthreads();
-    }
+    set_coefs<kDual>(A, vol, coef_vol, coef_s);
     const int l = l0 + min(g, nl - 1);
-    int c[3];
-    {
-      const int u = A.div_av.div(l);
-      c[A.au] = u;
-      c[A.av] = l - u * dv;
-      c[A.ax] = 0;
-    }
-    Ch ch0, ch1;
-    const bool sep0 = !id0 && A.ph[0].sep;
-    const bool sep1 = kDual && !id1 && A.ph[1].sep;
-    const PhaseCoef c0 = coef_s[0];
-    const PhaseCoef c1 = kDual ? coef_s[1] : PhaseCoef{0, 0, 0};
-    if (sep0) ch0.init(A.ph[0], c0, A.ph[0].rvec ? A.ph[0].rvec[c[A.ph[0].oaxis]] : 0.0, j, A.scale, A.scale_lo, G);
-    if (sep1) ch1.init(A.ph[1], c1, A.ph[1].rvec ? A.ph[1].rvec[c[A.ph[1].oaxis]] : 0.0, j, A.scale, A.scale_lo, G);
-    // V (element n = j + r R1 in slot r) times the factors of phase 0 or 1; which form applies
-    // (identity, line chirp, per-element evaluation) is decided once per line
-    auto factor0 = [&](float2 (&V)[R2]) {
-      if (id0) {
-#pragma unroll
-        for (int r = 0; r < R2; r++) V[r] = cscale2(V[r], A.scale, A.scale_lo);
-      } else if (sep0) {
-        ch0.apply(V);
-      } else {
-#pragma unroll
-        for (int r = 0; r < R2; r++) {
-          c[A.ax] = j + r * R1;
-          V[r] = cmul(V[r], phase_value(A.ph[0], c0, j + r * R1, c, A.scale, A.scale_lo));
-        }
-      }
-    };
-    auto factor1 = [&](float2 (&V)[R2]) {
-      if (id1) {
-#pragma unroll
-        for (int r = 0; r < R2; r++) V[r] = cscale2(V[r], A.scale, A.scale_lo);
-      } else if (sep1) {
-        ch1.apply(V);
-      } else {
-#pragma unroll
-        for (int r = 0; r < R2; r++) {
-          c[A.ax] = j + r * R1;
-          V[r] = cmul(V[r], phase_value(A.ph[1], c1, j + r * R1, c, A.scale, A.scale_lo));
-        }
-      }
-    };
-
-    float2* L0 = buf + g * LS;
-    float2* L1 = buf + (B + g) * LS;
-    float2 X[R2];
-    if (MODE == PM_INV) {
-      F::load_spectrum(L0, j, X);
-    } else {
-      F::forward(L0, j, X);
-    }
-    if (MODE == PM_DUAL_IN) {
-      float2 Y[R2];
-      F::forward(L1, j, Y);
-      if (j < R1) {
-        factor0(X);
-        factor1(Y);
-#pragma unroll
-        for (int r = 0; r < R2; r++) X[r] = cadd(X[r], Y[r]);
-      }
-      F::inverse(L0, j, X);
-    } else if (MODE == PM_DUAL_OUT) {
-      float2 Y[R2];
-      if (j < R1) {
-#pragma unroll
-        for (int r = 0; r < R2; r++) Y[r] = X[r];
-        factor0(X);
-        factor1(Y);
-      }
-      F::inverse(L0, j, X);
-      F::inverse(L1, j, Y);
-    } else {
-      if (j < R1) factor0(X);
-      if (MODE == PM_FWD) {
-        F::store_spectrum(L0, j, X);
-      } else {
-        F::inverse(L0, j, X);
-      }
-    }
+    const int u = A.div_av.div(l);
+    s0.line = tiles + cur * NT * TILE + g * PITCH;
+    s1.line = s0.line + TILE;
+    pass_line<N, MODE>(A, coef_s, u, l - u * dv, j, s0, s1, chirp_s[g]);
     __syncthreads();
-    // store the tile
-    const int nout = (MODE == PM_DUAL_OUT) ? 2 : 1;
-    for (int k = 0; k < nout; k++) {
-      float2* dst = (k == 0 ? A.out0 : A.out1) + (i64)vol * A.out_vs;
+#pragma unroll
+    for (int k = 0; k < (MODE == PM_DUAL_OUT ? 2 : 1); k++) {
+      if (cb >= nl) continue;
+      float2* dst = (k == 0 ? A.out0 : A.out1) + (i64)vol * A.out_vs + lb_s[cur][cb];
       const bool acc = (k == 0) && A.accum;
-      if (bfast) {
-        const int b = threadIdx.x % B;
-        if (b < nl) {
-          const i64 base = lb_s[cur][b];
-          const float2* s0 = buf + (k * B + b) * LS;
-          for (int n = threadIdx.x / B; n < N; n += 256 / B) {
-            float2 v = s0[n];
-            if (acc) v = cadd(v, dst[base + n * sa]);
-            dst[base + n * sa] = v;
-          }
-        }
-      } else {
-        const int b = threadIdx.x / G;
-        if (b < nl) {
-          const i64 base = lb_s[cur][b];
-          const float2* s0 = buf + (k * B + b) * LS;
-          for (int n = threadIdx.x % G; n < N; n += G) {
-            float2 v = s0[n];
-            if (acc) v = cadd(v, dst[base + n * sa]);
-            dst[base + n * sa] = v;
-          }
-        }
+      const float2* src = reinterpret_cast<const float2*>(tiles + (cur * NT + k) * TILE + cb * PITCH);
+      for (int n = cn; n < N; n += G) {
+        float2 v = src[n];
+        if (acc) v = cadd(v, dst[n * sa]);
+        dst[n * sa] = v;
       }
     }
     if (NBUF == 1) {
@@ -452,67 +279,77 @@ __global__ void __launch_bounds__(256, ME_PASS_MINB) fast_pass_kernel(const Pass
   cp_async_wait_all();
 }
 
-// ------------------------------------------------------------------ TMA tile staging
-// The same pass with each tile of B = 256 / G lines (16 lines of 16 threads, or 32 of 8) moved
-// by the TMA engine: one thread issues tiled tensor loads of the next tile (completing on an
-// mbarrier) and tiled tensor stores of the finished one, so no thread issues per-element global
-// loads or stores.  Used for the compile-time lengths when the lines of a tile are B
-// consecutive lines of one row (dims[av] a multiple of B) and every stride is a multiple of 16
-// bytes:
-//   strided lines (st[av] == 1): B / 16 sub-tiles [n][16 lines], each with the tensor map's
-//     128-byte swizzle (the 16-byte chunk index XOR n mod 8), so that the lanes of a line read
-//     and write distinct banks;
-//   contiguous lines (st[ax] == 1): tile [B lines][n], dense.
-// The FFT reads its line from the tile and hands its outputs back to the same places (a line
-// belongs to one thread group); its transposes use a padded scratch region per group.
+// ------------------------------------------------------------------ tiles on the TMA engine
+// The same pass with the tiles moved by the TMA engine, so that no thread issues per-element
+// global loads or stores (loads complete on an mbarrier):
+//   STRIDED (st[av] == 1): one tensor copy per tile and operand of up to 16 neighbouring lines of
+//     a row, [n][16 lines] with the tensor map's 128-byte swizzle; lines past the row's end read
+//     as zeros and are not written.  Needs base and strides that are multiples of 16 bytes.
+//   else (st[ax] == 1): each of a tile's lines is one bulk copy, issued by a lane of its own, into
+//     rows of line_pitch bytes.  Needs 16-byte aligned lines.
 struct PassTma {
   CUtensorMap in[2];
   CUtensorMap out[2];
   int in_rank[2];   // 3: one volume (or a broadcast input), 4: indexed by volume
   int out_rank[2];
+  FastDiv div_row;  // tiles per row of lines (strided)
+  int row_tiles;
 };
 
-template <int N, int B, bool STRIDED>
-__device__ __forceinline__ int tile_off(int b, int n) {
+// Tile position of work item tt of a volume: the first line's coordinates, and the lines in it.
+template <bool STRIDED>
+__device__ __forceinline__ void tile_coords(const PassArgs& A, const FastDiv& div_row,
+                                            int row_tiles, int tt, int& u, int& v0, int& nl) {
   if (STRIDED) {
-    const int sub = (B == 16) ? 0 : (b >> 4);  // 16-line sub-tile
-    const int bb = b & 15;
-    return sub * (16 * N * 8) + n * 128 + ((((bb >> 1) ^ n) & 7) << 4) + ((bb & 1) << 3);
+    u = div_row.div(tt);
+    v0 = (tt - u * row_tiles) * kTileLines;
+    nl = min(kTileLines, A.dims[A.av] - v0);
+  } else {
+    const int l0 = tt * kTileLines;
+    u = A.div_av.div(l0);
+    v0 = l0 - u * A.dims[A.av];
+    nl = min(kTileLines, A.nlines - l0);
   }
-  return (b * N + n) * 8;
 }
 
-template <int N, int R1, int R2, int MODE, bool STRIDED>
-__global__ void __launch_bounds__(256, ME_PASS_MINB)
+// Element offset of line b of a tile that starts at (u, v0) (contiguous lines; a tile may run
+// over into the next rows of lines).
+__device__ __forceinline__ i64 tile_line(const PassArgs& A, int u, int v0, int b) {
+  const int l = u * A.dims[A.av] + v0 + b;
+  const int ul = A.div_av.div(l);
+  return (i64)ul * A.st[A.au] + (i64)(l - ul * A.dims[A.av]) * A.st[A.av];
+}
+
+template <int N, bool STRIDED>
+struct TileShape {
+  static constexpr int PITCH = line_pitch(N);
+  static constexpr int TILE = STRIDED ? kTileLines * N * 8 : kTileLines * PITCH;
+};
+
+template <int N, int MODE, bool STRIDED>
+__global__ void __launch_bounds__(PassLine<N>::THREADS, pass_min_ctas(N, MODE != PM_SHEAR))
     tma_pass_kernel(const __grid_constant__ PassArgs A, const __grid_constant__ PassTma T) {
-  using F = LineFft<N, R1, R2>;
-  using Ch = LineChirp<N, R1, R2>;
-  constexpr int G = F::G;
-  constexpr int B = 256 / G;                      // lines per tile, one per thread group
-  constexpr int NSUB = STRIDED ? B / 16 : 1;       // tensor copies per tile and operand
-  constexpr int LS = F::LS;
-  constexpr bool kDual = (MODE == PM_DUAL_IN || MODE == PM_DUAL_OUT);
+  constexpr int G = PassLine<N>::G;
+  constexpr bool kDual = (MODE != PM_SHEAR);
   constexpr int NT = kDual ? 2 : 1;  // tiles per buffer
-  constexpr int NBUF = (kDual && ME_DUAL_SINGLE_BUFFER) ? 1 : 2;
+  constexpr int NBUF = kDual ? 1 : 2;
   constexpr int NIN = (MODE == PM_DUAL_IN) ? 2 : 1;
   constexpr int NOUT = (MODE == PM_DUAL_OUT) ? 2 : 1;
-  constexpr int TILE = B * N * 8;  // bytes; a multiple of 1024 for every length used here
-  constexpr int SUBT = TILE / NSUB;
-  static_assert(SUBT % 1024 == 0, "swizzled sub-tiles start on 1024-byte boundaries");
+  constexpr int PITCH = TileShape<N, STRIDED>::PITCH, TILE = TileShape<N, STRIDED>::TILE;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // the swizzle pattern repeats every 1024 bytes of shared-memory address
   unsigned char* tiles = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  float2* scratch = reinterpret_cast<float2*>(tiles + NBUF * NT * TILE);
   __shared__ __align__(8) uint64_t full[NBUF];
   __shared__ PhaseCoef coef_s[2];
 
-  const int tiles_per_vol = A.nlines / B;
+  const int tiles_per_vol = STRIDED ? T.row_tiles * A.dims[A.au] : (A.nlines + kTileLines - 1) / kTileLines;
   const int total = tiles_per_vol * A.nvol;
-  const int dv = A.dims[A.av];
-  const int g = threadIdx.x / G;
-  const int j = threadIdx.x % G;
-  const bool id0 = phase_is_identity(A.ph[0]);
-  const bool id1 = phase_is_identity(A.ph[1]);
+  int g, j;
+  line_place<G>(g, j);
+  __shared__ float2 chirp_s[kTileLines][2 * G];
+  Slots<G, STRIDED> s0, s1;
+  s0.init(g, j);
+  s1 = s0;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < NBUF; i++) mbar_init(&full[i], 1);
@@ -520,150 +357,78 @@ __global__ void __launch_bounds__(256, ME_PASS_MINB)
   }
   __syncthreads();
 
-  auto coords = [&](int t, int& vol, int& u, int& v0) {
-    vol = A.div_tiles.div(t);
-    const int l0 = (t - vol * tiles_per_vol) * B;
-    u = A.div_av.div(l0);
-    v0 = l0 - u * dv;
-  };
-  // thread 0: load work item t into buffer bufi, once the stores out of that buffer have read it
+  // warp 0: load work item t into buffer bufi, once the stores out of that buffer have read it
   auto issue = [&](int t, int bufi) {
-    int vol, u, v0;
-    coords(t, vol, u, v0);
+    const int vol = A.div_tiles.div(t);
+    int u, v0, nl;
+    tile_coords<STRIDED>(A, T.div_row, T.row_tiles, t - vol * tiles_per_vol, u, v0, nl);
     bulk_wait_read_all();
     fence_proxy_async_smem();
-    mbar_arrive_expect_tx(&full[bufi], NIN * TILE);
+    __syncwarp();
+    if (threadIdx.x == 0)
+      mbar_arrive_expect_tx(&full[bufi], NIN * (STRIDED ? TILE : nl * N * 8));
+    __syncwarp();
 #pragma unroll
     for (int k = 0; k < NIN; k++) {
-#pragma unroll
-      for (int q = 0; q < NSUB; q++) {
-        unsigned char* dst = tiles + (bufi * NT + k) * TILE + q * SUBT;
-        const int c0 = STRIDED ? v0 + 16 * q : 0, c1 = STRIDED ? 0 : v0;
-        if (T.in_rank[k] == 3) {
-          tma_load_3d(dst, &T.in[k], c0, c1, u, &full[bufi]);
-        } else {
-          tma_load_4d(dst, &T.in[k], c0, c1, u, vol, &full[bufi]);
+      unsigned char* dst = tiles + (bufi * NT + k) * TILE;
+      if (STRIDED) {
+        if (threadIdx.x == 0) {
+          if (T.in_rank[k] == 3) tma_load_3d(dst, &T.in[k], v0, 0, u, &full[bufi]);
+          else tma_load_4d(dst, &T.in[k], v0, 0, u, vol, &full[bufi]);
         }
+      } else if ((int)threadIdx.x < nl) {
+        bulk_g2s(dst + threadIdx.x * PITCH,
+                 (k == 0 ? A.in0 : A.in1) + (i64)vol * A.in_vs + tile_line(A, u, v0, threadIdx.x),
+                 N * 8, &full[bufi]);
       }
     }
   };
 
-  if (threadIdx.x == 0 && (int)blockIdx.x < total) issue(blockIdx.x, 0);
+  const bool mover = threadIdx.x < 32;
+  if (mover && (int)blockIdx.x < total) issue(blockIdx.x, 0);
   int coef_vol = -1;
   int it = 0;
   for (int t = blockIdx.x; t < total; t += gridDim.x, it++) {
     const int cur = (NBUF == 2) ? (it & 1) : 0;
     const unsigned parity = (NBUF == 2) ? ((it >> 1) & 1) : (it & 1);
-    int vol, u, v0;
-    coords(t, vol, u, v0);
+    const int vol = A.div_tiles.div(t);
+    int u, v0, nl;
+    tile_coords<STRIDED>(A, T.div_row, T.row_tiles, t - vol * tiles_per_vol, u, v0, nl);
     mbar_wait_bounded(&full[cur], parity, WF_LINE_PASS);
-    if (NBUF == 2 && threadIdx.x == 0 && t + (int)gridDim.x < total) issue(t + gridDim.x, cur ^ 1);
-    // the shear coefficients depend on the volume only (the barrier before the previous
-    // tile's store separates every read of coef_s from this write)
-    if (vol != coef_vol) {
-      if (threadIdx.x < (kDual ? 2 : 1)) {
-        PhaseCoef cf{0, 0, 0};
-        if (A.params) cf = phase_coef(A.ph[threadIdx.x], A.params + (i64)vol * A.pstride, A.ax);
-        coef_s[threadIdx.x] = cf;
-      }
-      coef_vol = vol;
-      __syncthreads();
+    if (NBUF == 2 && mover && t + (int)gridDim.x < total) issue(t + gridDim.x, cur ^ 1);
+    // (the barrier before the previous tile's store separates every read of coef_s from a write)
+    set_coefs<kDual>(A, vol, coef_vol, coef_s);
+    int ul = u, vl = v0 + min(g, nl - 1);
+    if (!STRIDED) {
+      const int l = u * A.dims[A.av] + vl;
+      ul = A.div_av.div(l);
+      vl = l - ul * A.dims[A.av];
     }
-    int c[3];
-    c[A.au] = u;
-    c[A.av] = v0 + g;
-    c[A.ax] = 0;
-    Ch ch0, ch1;
-    const bool sep0 = !id0 && A.ph[0].sep;
-    const bool sep1 = kDual && !id1 && A.ph[1].sep;
-    const PhaseCoef c0 = coef_s[0];
-    const PhaseCoef c1 = kDual ? coef_s[1] : PhaseCoef{0, 0, 0};
-    if (sep0) ch0.init(A.ph[0], c0, A.ph[0].rvec ? A.ph[0].rvec[c[A.ph[0].oaxis]] : 0.0, j, A.scale, A.scale_lo, G);
-    if (sep1) ch1.init(A.ph[1], c1, A.ph[1].rvec ? A.ph[1].rvec[c[A.ph[1].oaxis]] : 0.0, j, A.scale, A.scale_lo, G);
-    auto factor0 = [&](float2 (&V)[R2]) {
-      if (id0) {
-#pragma unroll
-        for (int r = 0; r < R2; r++) V[r] = cscale2(V[r], A.scale, A.scale_lo);
-      } else if (sep0) {
-        ch0.apply(V);
-      } else {
-#pragma unroll
-        for (int r = 0; r < R2; r++) {
-          c[A.ax] = j + r * R1;
-          V[r] = cmul(V[r], phase_value(A.ph[0], c0, j + r * R1, c, A.scale, A.scale_lo));
-        }
-      }
-    };
-    auto factor1 = [&](float2 (&V)[R2]) {
-      if (id1) {
-#pragma unroll
-        for (int r = 0; r < R2; r++) V[r] = cscale2(V[r], A.scale, A.scale_lo);
-      } else if (sep1) {
-        ch1.apply(V);
-      } else {
-#pragma unroll
-        for (int r = 0; r < R2; r++) {
-          c[A.ax] = j + r * R1;
-          V[r] = cmul(V[r], phase_value(A.ph[1], c1, j + r * R1, c, A.scale, A.scale_lo));
-        }
-      }
-    };
-
-    unsigned char* tb0 = tiles + (cur * NT) * TILE;
-    unsigned char* tb1 = tiles + (cur * NT + 1) * TILE;
-    auto load0 = [&](int n) { return *reinterpret_cast<const float2*>(tb0 + tile_off<N, B, STRIDED>(g, n)); };
-    auto load1 = [&](int n) { return *reinterpret_cast<const float2*>(tb1 + tile_off<N, B, STRIDED>(g, n)); };
-    auto store0 = [&](int, int n, float2 v) { *reinterpret_cast<float2*>(tb0 + tile_off<N, B, STRIDED>(g, n)) = v; };
-    auto store1 = [&](int, int n, float2 v) { *reinterpret_cast<float2*>(tb1 + tile_off<N, B, STRIDED>(g, n)) = v; };
-    float2* L = scratch + g * LS;
-    float2 X[R2];
-    F::forward_from(load0, L, j, X);
-    if (MODE == PM_DUAL_IN) {
-      float2 Y[R2];
-      F::forward_from(load1, L, j, Y);
-      if (j < R1) {
-        factor0(X);
-        factor1(Y);
-#pragma unroll
-        for (int r = 0; r < R2; r++) X[r] = cadd(X[r], Y[r]);
-      }
-      F::inverse_to(L, j, X, store0);
-    } else if (MODE == PM_DUAL_OUT) {
-      float2 Y[R2];
-      if (j < R1) {
-#pragma unroll
-        for (int r = 0; r < R2; r++) Y[r] = X[r];
-        factor0(X);
-        factor1(Y);
-      }
-      F::inverse_to(L, j, X, store0);
-      F::inverse_to(L, j, Y, store1);
-    } else {
-      if (j < R1) factor0(X);
-      F::inverse_to(L, j, X, store0);
-    }
+    s0.line = tiles + cur * NT * TILE + (STRIDED ? 0 : g * PITCH);
+    s1.line = s0.line + TILE;
+    pass_line<N, MODE>(A, coef_s, ul, vl, j, s0, s1, chirp_s[g]);
     // the tile's generic-proxy writes are ordered before the async-proxy store
     fence_proxy_async_smem();
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (mover) {
 #pragma unroll
       for (int k = 0; k < NOUT; k++) {
-#pragma unroll
-        for (int q = 0; q < NSUB; q++) {
-          const unsigned char* src = tiles + (cur * NT + k) * TILE + q * SUBT;
-          const int c0s = STRIDED ? v0 + 16 * q : 0, c1s = STRIDED ? 0 : v0;
-          if (T.out_rank[k] == 3) {
-            tma_store_3d(&T.out[k], src, c0s, c1s, u);
-          } else {
-            tma_store_4d(&T.out[k], src, c0s, c1s, u, vol);
+        const unsigned char* src = tiles + (cur * NT + k) * TILE;
+        if (STRIDED) {
+          if (threadIdx.x == 0) {
+            if (T.out_rank[k] == 3) tma_store_3d(&T.out[k], src, v0, 0, u);
+            else tma_store_4d(&T.out[k], src, v0, 0, u, vol);
           }
+        } else if ((int)threadIdx.x < nl) {
+          bulk_s2g((k == 0 ? A.out0 : A.out1) + (i64)vol * A.out_vs + tile_line(A, u, v0, threadIdx.x),
+                   src + threadIdx.x * PITCH, N * 8);
         }
       }
       bulk_commit();
       if (NBUF == 1 && t + (int)gridDim.x < total) issue(t + gridDim.x, 0);
     }
   }
-  if (threadIdx.x == 0) bulk_wait_all();
+  if (mover) bulk_wait_all();
 }
 
 // ME_NO_TMA=1 in the environment keeps every pass on the cp.async kernel (for comparisons).
@@ -689,58 +454,38 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
-// Tensor map of one operand of a TMA pass (8-byte elements; boxes of 16 strided lines or of B
-// contiguous lines); rank 3 when the operand is one volume, else rank 4 with the volume index
-// outermost.
-static bool encode_pass_map(CUtensorMap* m, const void* base, const PassArgs& A, bool strided,
-                            i64 vs, int rank, int B) {
+// Tensor map of one operand of a strided TMA pass (8-byte elements, boxes of 16 lines); rank 3
+// when the operand is one volume, else rank 4 with the volume index outermost.
+static bool encode_pass_map(CUtensorMap* m, const void* base, const PassArgs& A, i64 vs, int rank) {
   PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
   if (!enc) return false;
-  const int N = A.dims[A.ax];
-  cuuint64_t dims[4];
-  cuuint64_t strides[3];
-  cuuint32_t box[4];
+  const cuuint64_t dims[4] = {(cuuint64_t)A.dims[A.av], (cuuint64_t)A.dims[A.ax],
+                              (cuuint64_t)A.dims[A.au], (cuuint64_t)A.nvol};
+  const cuuint64_t strides[3] = {(cuuint64_t)A.st[A.ax] * 8, (cuuint64_t)A.st[A.au] * 8,
+                                 (cuuint64_t)vs * 8};
+  const cuuint32_t box[4] = {kTileLines, (cuuint32_t)A.dims[A.ax], 1, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
-  if (strided) {
-    dims[0] = (cuuint64_t)A.dims[A.av];
-    dims[1] = (cuuint64_t)N;
-    strides[0] = (cuuint64_t)A.st[A.ax] * 8;
-    box[0] = 16;
-    box[1] = (cuuint32_t)N;
-  } else {
-    dims[0] = (cuuint64_t)N;
-    dims[1] = (cuuint64_t)A.dims[A.av];
-    strides[0] = (cuuint64_t)A.st[A.av] * 8;
-    box[0] = (cuuint32_t)N;
-    box[1] = (cuuint32_t)B;
-  }
-  dims[2] = (cuuint64_t)A.dims[A.au];
-  strides[1] = (cuuint64_t)A.st[A.au] * 8;
-  box[2] = 1;
-  dims[3] = (cuuint64_t)A.nvol;
-  strides[2] = (cuuint64_t)vs * 8;
-  box[3] = 1;
   const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT64, (cuuint32_t)rank,
                          const_cast<void*>(base), dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         strided ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
 
-// Whether pass A (mode, tiles of B lines) can run on the TMA kernel; fills the tensor maps.
-static bool tma_pass_setup(int mode, const PassArgs& A, int B, bool* strided, PassTma* T) {
+// Whether pass A can run on the TMA kernel, and then how: strided or contiguous lines, the
+// tensor maps of the former.  All strides have to be even (16 bytes) and all bases aligned.
+static bool tma_pass_setup(int mode, const PassArgs& A, bool* strided, PassTma* T) {
   if (!tma_passes_enabled()) return false;
   if (mode != PM_SHEAR && mode != PM_DUAL_OUT && mode != PM_DUAL_IN) return false;
   if (A.accum) return false;
-  const int dv = A.dims[A.av];
-  if (dv % B != 0) return false;
   const bool s = (A.st[A.av] == 1);
   if (!s && A.st[A.ax] != 1) return false;
   const i64 other = s ? A.st[A.ax] : A.st[A.av];
   if (other % 2 != 0 || A.st[A.au] % 2 != 0) return false;
   const i64 lim = (i64)1 << 36;  // strides below 2^40 bytes
   if (other >= lim || A.st[A.au] >= lim || A.in_vs >= lim || A.out_vs >= lim) return false;
+  // tiles of fewer than eight lines in use are better packed by the cp.async kernel
+  if (s && A.dims[A.av] % kTileLines != 0 && A.dims[A.av] < 2 * kTileLines) return false;
   const int nin = (mode == PM_DUAL_IN) ? 2 : 1, nout = (mode == PM_DUAL_OUT) ? 2 : 1;
   const float2* ins[2] = {A.in0, A.in1};
   float2* outs[2] = {A.out0, A.out1};
@@ -749,90 +494,89 @@ static bool tma_pass_setup(int mode, const PassArgs& A, int B, bool* strided, Pa
     const bool one = (A.in_vs == 0 || A.nvol == 1);
     if (!one && A.in_vs % 2 != 0) return false;
     T->in_rank[k] = one ? 3 : 4;
-    if (!encode_pass_map(&T->in[k], ins[k], A, s, A.in_vs, T->in_rank[k], B)) return false;
+    if (s && !encode_pass_map(&T->in[k], ins[k], A, A.in_vs, T->in_rank[k])) return false;
   }
   for (int k = 0; k < nout; k++) {
     if ((uintptr_t)outs[k] % 16 != 0) return false;
     const bool one = (A.nvol == 1);
     if (!one && A.out_vs % 2 != 0) return false;
     T->out_rank[k] = one ? 3 : 4;
-    if (!encode_pass_map(&T->out[k], outs[k], A, s, A.out_vs, T->out_rank[k], B)) return false;
+    if (s && !encode_pass_map(&T->out[k], outs[k], A, A.out_vs, T->out_rank[k])) return false;
   }
+  T->row_tiles = s ? (A.dims[A.av] + kTileLines - 1) / kTileLines : 1;
+  T->div_row.set(T->row_tiles);
   *strided = s;
   return true;
 }
 
-template <int N, int R1, int R2, int MODE, bool STRIDED>
-static int launch_tma(PassArgs& A, const PassTma& T, cudaStream_t stream) {
-  using F = LineFft<N, R1, R2>;
-  constexpr bool kDual = (MODE == PM_DUAL_IN || MODE == PM_DUAL_OUT);
-  constexpr int NBUF = (kDual && ME_DUAL_SINGLE_BUFFER) ? 1 : 2;
-  constexpr int B = 256 / F::G;
-  const size_t smem = 1024 + (size_t)NBUF * (kDual ? 2 : 1) * B * N * 8 +
-                      sizeof(float2) * (size_t)F::LS * B;
-  A.div_tiles.set(A.nlines / B);
-  auto kern = tma_pass_kernel<N, R1, R2, MODE, STRIDED>;
-  const int rc = check_cuda(allow_smem(kern, smem), "tma pass smem");
-  if (rc != ME_OK) return rc;
-  static int occ[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+// Work items of a volume.
+static int tiles_of(const PassArgs& A, bool strided_tma) {
+  return strided_tma ? (A.dims[A.av] + kTileLines - 1) / kTileLines * A.dims[A.au]
+                     : (A.nlines + kTileLines - 1) / kTileLines;
+}
+
+// Persistent grid of a kernel: all resident CTAs, or fewer where there are fewer tiles.  `occ`
+// keeps the device's resident CTAs for the kernel (one launch shape per instantiation).
+template <typename K>
+static int pass_grid(K kern, int threads, size_t smem, long long tiles, std::atomic<int> (&occ)[8]) {
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 8 && occ[dev] == 0) {
-    int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, 256, smem);
-    int sms = 0;
+  int res = dev < 8 ? occ[dev].load(std::memory_order_relaxed) : 0;
+  if (res == 0) {
+    int nb = 0, sms = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, threads, smem);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    occ[dev] = std::max(1, nb) * std::max(1, sms);
+    res = std::max(1, nb) * std::max(1, sms);
+    if (dev < 8) occ[dev].store(res, std::memory_order_relaxed);
   }
-  const long long tiles = (long long)(A.nlines / B) * A.nvol;
-  const int grid = (int)std::min<long long>(tiles, dev < 8 ? occ[dev] : 148 * 2);
+  return (int)std::min<long long>(tiles, res);
+}
+
+template <int N, int MODE, bool STRIDED>
+static int launch_tma(PassArgs& A, const PassTma& T, cudaStream_t stream) {
+  const size_t smem = 1024 + 2 * (size_t)TileShape<N, STRIDED>::TILE;
+  const int tiles = tiles_of(A, STRIDED);
+  A.div_tiles.set(tiles);
+  auto kern = tma_pass_kernel<N, MODE, STRIDED>;
+  const int rc = check_cuda(allow_smem(kern, smem), "tma pass smem");
+  if (rc != ME_OK) return rc;
+  static std::atomic<int> occ[8];
+  const int grid = pass_grid(kern, PassLine<N>::THREADS, smem, (long long)tiles * A.nvol, occ);
   count_launch();
-  kern<<<grid, 256, smem, stream>>>(A, T);
+  kern<<<grid, PassLine<N>::THREADS, smem, stream>>>(A, T);
   return check_cuda(cudaGetLastError(), "tma pass launch");
 }
 
-template <int N, int R1, int R2, int MODE>
+template <int N, int MODE>
 static int launch_fast(PassArgs& A, cudaStream_t stream) {
-  using F = LineFft<N, R1, R2>;
   if constexpr (MODE == PM_SHEAR || MODE == PM_DUAL_OUT || MODE == PM_DUAL_IN) {
     PassTma T;
     bool strided = false;
-    if (tma_pass_setup(MODE, A, 256 / F::G, &strided, &T))
-      return strided ? launch_tma<N, R1, R2, MODE, true>(A, T, stream)
-                     : launch_tma<N, R1, R2, MODE, false>(A, T, stream);
+    if (tma_pass_setup(MODE, A, &strided, &T))
+      return strided ? launch_tma<N, MODE, true>(A, T, stream)
+                     : launch_tma<N, MODE, false>(A, T, stream);
   }
-  constexpr int B = 256 / F::G;
-  constexpr bool kDual = (MODE == PM_DUAL_IN || MODE == PM_DUAL_OUT);
-  const size_t smem = sizeof(float2) * (size_t)F::LS * B * (kDual ? 2 : 1) *
-                      ((kDual && ME_DUAL_SINGLE_BUFFER) ? 1 : 2);
-  A.div_tiles.set((A.nlines + B - 1) / B);
-  const int rc = check_cuda(allow_smem(fast_pass_kernel<N, R1, R2, MODE>, smem), "pass smem");
+  const size_t smem = 2 * (size_t)kTileLines * line_pitch(N);
+  const int tiles = tiles_of(A, false);
+  A.div_tiles.set(tiles);
+  auto kern = fast_pass_kernel<N, MODE>;
+  const int rc = check_cuda(allow_smem(kern, smem), "pass smem");
   if (rc != ME_OK) return rc;
-  static int occ[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 8 && occ[dev] == 0) {
-    int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fast_pass_kernel<N, R1, R2, MODE>, 256, smem);
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    occ[dev] = std::max(1, nb) * std::max(1, sms);
-  }
-  const long long tiles = (long long)((A.nlines + B - 1) / B) * A.nvol;
-  const int grid = (int)std::min<long long>(tiles, dev < 8 ? occ[dev] : 148 * 2);
+  static std::atomic<int> occ[8];
+  const int grid = pass_grid(kern, PassLine<N>::THREADS, smem, (long long)tiles * A.nvol, occ);
   count_launch();
-  fast_pass_kernel<N, R1, R2, MODE><<<grid, 256, smem, stream>>>(A);
+  kern<<<grid, PassLine<N>::THREADS, smem, stream>>>(A);
   return check_cuda(cudaGetLastError(), "fast pass launch");
 }
 
-template <int N, int R1, int R2>
+template <int N>
 static int launch_fast_mode(int mode, PassArgs& A, cudaStream_t stream) {
   switch (mode) {
-    case PM_SHEAR: return launch_fast<N, R1, R2, PM_SHEAR>(A, stream);
-    case PM_DUAL_OUT: return launch_fast<N, R1, R2, PM_DUAL_OUT>(A, stream);
-    case PM_DUAL_IN: return launch_fast<N, R1, R2, PM_DUAL_IN>(A, stream);
-    case PM_FWD: return launch_fast<N, R1, R2, PM_FWD>(A, stream);
-    default: return launch_fast<N, R1, R2, PM_INV>(A, stream);
+    case PM_SHEAR: return launch_fast<N, PM_SHEAR>(A, stream);
+    case PM_DUAL_OUT: return launch_fast<N, PM_DUAL_OUT>(A, stream);
+    case PM_DUAL_IN: return launch_fast<N, PM_DUAL_IN>(A, stream);
+    case PM_FWD: return launch_fast<N, PM_FWD>(A, stream);
+    default: return launch_fast<N, PM_INV>(A, stream);
   }
 }
 
@@ -840,7 +584,7 @@ static int launch_fast_mode(int mode, PassArgs& A, cudaStream_t stream) {
 static int try_fast(int mode, PassArgs& A, cudaStream_t stream) {
   switch (A.plan.n) {
 #define ME_FAST_CASE(N, R1, R2) \
-  case N: return launch_fast_mode<N, R1, R2>(mode, A, stream);
+  case N: return launch_fast_mode<N>(mode, A, stream);
     ME_FAST_LENGTHS(ME_FAST_CASE)
 #undef ME_FAST_CASE
     default: return -1;
@@ -960,59 +704,54 @@ struct MultiPassArgs {
   PassArgs job[kMaxMultiJobs];
 };
 
-template <int N, int R1, int R2>
-__global__ void __launch_bounds__(256, ME_PASS_MINB)
+template <int N>
+__global__ void __launch_bounds__(PassLine<N>::THREADS, pass_min_ctas(N, false))
     multi_shear_kernel(const __grid_constant__ MultiPassArgs M) {
-  using F = LineFft<N, R1, R2>;
-  using Ch = LineChirp<N, R1, R2>;
-  constexpr int G = F::G;
-  constexpr int B = 256 / G;
-  constexpr int LS = F::LS;
-  extern __shared__ __align__(16) float2 smem[];
-  __shared__ i64 lb_s[2][B];  // line base offsets of the tile in each buffer
-  __shared__ PhaseCoef coef_s;
+  constexpr int G = PassLine<N>::G, B = kTileLines;
+  constexpr int PITCH = line_pitch(N), TILE = B * PITCH;
+  extern __shared__ __align__(128) unsigned char tiles[];
+  __shared__ PhaseCoef coef_s[2];
   const int total = M.tile_off[M.njobs];
-  const int g = threadIdx.x / G;
-  const int j = threadIdx.x % G;
+  int g, j;
+  line_place<G>(g, j);
+  __shared__ float2 chirp_s[kTileLines][2 * G];
+  Slots<G, false> s0;
+  s0.init(g, j);
   auto job_of = [&](int t) {
     int k = 0;
     while (k + 1 < M.njobs && t >= M.tile_off[k + 1]) k++;
     return k;
   };
+  // a work item's volume, first line and lines, and this thread's place when it copies
+  struct Item {
+    int vol, l0, nl, cb, cn;
+    i64 base;
+  };
+  auto item = [&](const PassArgs& A, int tt) {
+    Item I;
+    const int tiles_per_vol = (A.nlines + B - 1) / B;
+    I.vol = A.div_tiles.div(tt);
+    I.l0 = (tt - I.vol * tiles_per_vol) * B;
+    I.nl = min(B, A.nlines - I.l0);
+    const bool bfast = (A.st[A.av] == 1);
+    I.cb = bfast ? threadIdx.x % B : threadIdx.x / G;
+    I.cn = bfast ? threadIdx.x / B : threadIdx.x % G;
+    const int l = I.l0 + min(I.cb, I.nl - 1);
+    const int u = A.div_av.div(l);
+    I.base = (i64)u * A.st[A.au] + (i64)(l - u * A.dims[A.av]) * A.st[A.av];
+    return I;
+  };
   // issue the loads of work item t into buffer `bufi` (the caller has synchronised)
   auto issue = [&](int t, int bufi) {
     const int k = job_of(t);
     const PassArgs& A = M.job[k];
-    const int tt = t - M.tile_off[k];
-    const int tiles_per_vol = (A.nlines + B - 1) / B;
-    const int vol = A.div_tiles.div(tt);
-    const int l0 = (tt - vol * tiles_per_vol) * B;
-    const int nl = min(B, A.nlines - l0);
+    const Item I = item(A, t - M.tile_off[k]);
     const i64 sa = A.st[A.ax];
-    const int dv = A.dims[A.av];
-    auto line_base = [&](int l) {
-      const int u = A.div_av.div(l);
-      return (i64)u * A.st[A.au] + (i64)(l - u * dv) * A.st[A.av];
-    };
-    float2* buf = smem + bufi * B * LS;
-    if (threadIdx.x < B) lb_s[bufi][threadIdx.x] = line_base(l0 + min((int)threadIdx.x, nl - 1));
-    const float2* src = A.in0 + (i64)vol * A.in_vs;
-    if (A.st[A.av] == 1) {
-      const int b = threadIdx.x % B;
-      const i64 base = line_base(l0 + min(b, nl - 1));
-      float2* dst0 = buf + b * LS;
-      for (int n = threadIdx.x / B; n < N; n += 256 / B) {
-        if (b < nl) cp_async8(dst0 + n, src + base + n * sa);
-        else dst0[n] = make_float2(0.f, 0.f);
-      }
-    } else {
-      const int b = threadIdx.x / G;
-      const i64 base = line_base(l0 + min(b, nl - 1));
-      float2* dst0 = buf + b * LS;
-      for (int n = threadIdx.x % G; n < N; n += G) {
-        if (b < nl) cp_async8(dst0 + n, src + base + n * sa);
-        else dst0[n] = make_float2(0.f, 0.f);
-      }
+    const float2* src = A.in0 + (i64)I.vol * A.in_vs + I.base;
+    float2* dst = reinterpret_cast<float2*>(tiles + bufi * TILE + I.cb * PITCH);
+    for (int n = I.cn; n < N; n += G) {
+      if (I.cb < I.nl) cp_async8(dst + n, src + n * sa);
+      else dst[n] = make_float2(0.f, 0.f);
     }
     cp_async_commit();
   };
@@ -1022,87 +761,39 @@ __global__ void __launch_bounds__(256, ME_PASS_MINB)
   for (int t = blockIdx.x; t < total; t += gridDim.x) {
     const int k = job_of(t);
     const PassArgs& A = M.job[k];
-    const int tt = t - M.tile_off[k];
-    const int tiles_per_vol = (A.nlines + B - 1) / B;
-    const int vol = A.div_tiles.div(tt);
-    const int l0 = (tt - vol * tiles_per_vol) * B;
-    const int nl = min(B, A.nlines - l0);
+    const Item I = item(A, t - M.tile_off[k]);
     cp_async_wait_all();
     __syncthreads();
     if (t + (int)gridDim.x < total) issue(t + gridDim.x, cur ^ 1);
-    float2* buf = smem + cur * B * LS;
-    // the shear coefficients depend on the job and volume only (both uniform over the CTA)
-    if (k != coef_job || vol != coef_vol) {
-      if (threadIdx.x == 0) {
-        PhaseCoef cf{0, 0, 0};
-        if (A.params) cf = phase_coef(A.ph[0], A.params + (i64)vol * A.pstride, A.ax);
-        coef_s = cf;
-      }
-      coef_job = k;
-      coef_vol = vol;
-      __syncthreads();
-    }
-    const bool id0 = phase_is_identity(A.ph[0]);
-    const int dv = A.dims[A.av];
-    const int l = l0 + min(g, nl - 1);
-    int c[3];
-    {
-      const int u = A.div_av.div(l);
-      c[A.au] = u;
-      c[A.av] = l - u * dv;
-      c[A.ax] = 0;
-    }
-    const bool sep0 = !id0 && A.ph[0].sep;
-    const PhaseCoef c0 = coef_s;
-    Ch ch0;
-    if (sep0) ch0.init(A.ph[0], c0, A.ph[0].rvec ? A.ph[0].rvec[c[A.ph[0].oaxis]] : 0.0, j, A.scale, A.scale_lo, G);
-    float2* L0 = buf + g * LS;
-    float2 X[R2];
-    F::forward(L0, j, X);
-    if (j < R1) {
-      if (id0) {
-#pragma unroll
-        for (int r = 0; r < R2; r++) X[r] = cscale2(X[r], A.scale, A.scale_lo);
-      } else if (sep0) {
-        ch0.apply(X);
-      } else {
-#pragma unroll
-        for (int r = 0; r < R2; r++) {
-          c[A.ax] = j + r * R1;
-          X[r] = cmul(X[r], phase_value(A.ph[0], c0, j + r * R1, c, A.scale, A.scale_lo));
-        }
-      }
-    }
-    F::inverse(L0, j, X);
+    if (k != coef_job) coef_vol = -1;
+    coef_job = k;
+    set_coefs<false>(A, I.vol, coef_vol, coef_s);
+    const int l = I.l0 + min(g, I.nl - 1);
+    const int u = A.div_av.div(l);
+    s0.line = tiles + cur * TILE + g * PITCH;
+    pass_line<N, PM_SHEAR>(A, coef_s, u, l - u * A.dims[A.av], j, s0, s0, chirp_s[g]);
     __syncthreads();
-    float2* dst = A.out0 + (i64)vol * A.out_vs;
-    const i64 sa = A.st[A.ax];
-    if (A.st[A.av] == 1) {
-      const int b = threadIdx.x % B;
-      if (b < nl) {
-        const float2* s0 = buf + b * LS;
-        for (int n = threadIdx.x / B; n < N; n += 256 / B) dst[lb_s[cur][b] + n * sa] = s0[n];
-      }
-    } else {
-      const int b = threadIdx.x / G;
-      if (b < nl) {
-        const float2* s0 = buf + b * LS;
-        for (int n = threadIdx.x % G; n < N; n += G) dst[lb_s[cur][b] + n * sa] = s0[n];
-      }
+    if (I.cb < I.nl) {
+      const i64 sa = A.st[A.ax];
+      float2* dst = A.out0 + (i64)I.vol * A.out_vs + I.base;
+      const float2* src = reinterpret_cast<const float2*>(tiles + cur * TILE + I.cb * PITCH);
+      for (int n = I.cn; n < N; n += G) dst[n * sa] = src[n];
     }
     cur ^= 1;
   }
   cp_async_wait_all();
 }
 
-// The multi-job shear step on TMA tiles: the tiles of every job move by tensor loads and
-// stores, as in tma_pass_kernel, through each job's own tensor maps.  Used when every job of
-// the launch qualifies for tma_pass_kernel with the same tile layout (all strided or all
-// contiguous, as the jobs of one shear step in the same volume layout are).
+// The multi-job shear step on TMA tiles: the tiles of every job move as in tma_pass_kernel,
+// through each job's own tensor maps.  Used when every job of the launch qualifies for
+// tma_pass_kernel with the same tile layout (all strided or all contiguous, as the jobs of one
+// shear step in the same volume layout are).
 struct MultiTmaJob {
   CUtensorMap in;
   CUtensorMap out;
   int in_rank, out_rank;
+  FastDiv div_row;
+  int row_tiles;
 };
 
 struct MultiTmaArgs {
@@ -1112,26 +803,21 @@ struct MultiTmaArgs {
   MultiTmaJob tm[kMaxMultiJobs];
 };
 
-template <int N, int R1, int R2, bool STRIDED>
-__global__ void __launch_bounds__(256, ME_PASS_MINB)
+template <int N, bool STRIDED>
+__global__ void __launch_bounds__(PassLine<N>::THREADS, pass_min_ctas(N, false))
     tma_multi_shear_kernel(const __grid_constant__ MultiTmaArgs M) {
-  using F = LineFft<N, R1, R2>;
-  using Ch = LineChirp<N, R1, R2>;
-  constexpr int G = F::G;
-  constexpr int B = 256 / G;
-  constexpr int LS = F::LS;
-  constexpr int TILE = B * N * 8;
-  constexpr int NSUB = STRIDED ? B / 16 : 1;
-  constexpr int SUBT = TILE / NSUB;
-  static_assert(SUBT % 1024 == 0, "swizzled sub-tiles start on 1024-byte boundaries");
+  constexpr int G = PassLine<N>::G;
+  constexpr int PITCH = TileShape<N, STRIDED>::PITCH, TILE = TileShape<N, STRIDED>::TILE;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char* tiles = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  float2* scratch = reinterpret_cast<float2*>(tiles + 2 * TILE);
   __shared__ __align__(8) uint64_t full[2];
-  __shared__ PhaseCoef coef_s;
+  __shared__ PhaseCoef coef_s[2];
   const int total = M.tile_off[M.njobs];
-  const int g = threadIdx.x / G;
-  const int j = threadIdx.x % G;
+  int g, j;
+  line_place<G>(g, j);
+  __shared__ float2 chirp_s[kTileLines][2 * G];
+  Slots<G, STRIDED> s0;
+  s0.init(g, j);
   if (threadIdx.x == 0) {
     mbar_init(&full[0], 1);
     mbar_init(&full[1], 1);
@@ -1143,36 +829,40 @@ __global__ void __launch_bounds__(256, ME_PASS_MINB)
     while (k + 1 < M.njobs && t >= M.tile_off[k + 1]) k++;
     return k;
   };
-  auto coords = [&](int k, int t, int& vol, int& u, int& v0) {
+  auto coords = [&](int k, int t, int& vol, int& u, int& v0, int& nl) {
     const PassArgs& A = M.job[k];
+    const MultiTmaJob& J = M.tm[k];
+    const int per_vol = STRIDED ? J.row_tiles * A.dims[A.au] : (A.nlines + kTileLines - 1) / kTileLines;
     const int tt = t - M.tile_off[k];
     vol = A.div_tiles.div(tt);
-    const int l0 = (tt - vol * (A.nlines / B)) * B;
-    u = A.div_av.div(l0);
-    v0 = l0 - u * A.dims[A.av];
+    tile_coords<STRIDED>(A, J.div_row, J.row_tiles, tt - vol * per_vol, u, v0, nl);
   };
-  // thread 0: load work item t into buffer bufi, once the stores out of that buffer have read it
+  // warp 0: load work item t into buffer bufi, once the stores out of that buffer have read it
   auto issue = [&](int t, int bufi) {
     const int k = job_of(t);
-    int vol, u, v0;
-    coords(k, t, vol, u, v0);
+    int vol, u, v0, nl;
+    coords(k, t, vol, u, v0, nl);
+    const PassArgs& A = M.job[k];
     const MultiTmaJob& J = M.tm[k];
     bulk_wait_read_all();
     fence_proxy_async_smem();
-    mbar_arrive_expect_tx(&full[bufi], TILE);
-#pragma unroll
-    for (int q = 0; q < NSUB; q++) {
-      unsigned char* dst = tiles + bufi * TILE + q * SUBT;
-      const int c0 = STRIDED ? v0 + 16 * q : 0, c1 = STRIDED ? 0 : v0;
-      if (J.in_rank == 3) {
-        tma_load_3d(dst, &J.in, c0, c1, u, &full[bufi]);
-      } else {
-        tma_load_4d(dst, &J.in, c0, c1, u, vol, &full[bufi]);
+    __syncwarp();
+    if (threadIdx.x == 0) mbar_arrive_expect_tx(&full[bufi], STRIDED ? TILE : nl * N * 8);
+    __syncwarp();
+    unsigned char* dst = tiles + bufi * TILE;
+    if (STRIDED) {
+      if (threadIdx.x == 0) {
+        if (J.in_rank == 3) tma_load_3d(dst, &J.in, v0, 0, u, &full[bufi]);
+        else tma_load_4d(dst, &J.in, v0, 0, u, vol, &full[bufi]);
       }
+    } else if ((int)threadIdx.x < nl) {
+      bulk_g2s(dst + threadIdx.x * PITCH,
+               A.in0 + (i64)vol * A.in_vs + tile_line(A, u, v0, threadIdx.x), N * 8, &full[bufi]);
     }
   };
 
-  if (threadIdx.x == 0 && (int)blockIdx.x < total) issue(blockIdx.x, 0);
+  const bool mover = threadIdx.x < 32;
+  if (mover && (int)blockIdx.x < total) issue(blockIdx.x, 0);
   int coef_job = -1, coef_vol = -1;
   int it = 0;
   for (int t = blockIdx.x; t < total; t += gridDim.x, it++) {
@@ -1180,106 +870,65 @@ __global__ void __launch_bounds__(256, ME_PASS_MINB)
     const int k = job_of(t);
     const PassArgs& A = M.job[k];
     const MultiTmaJob& J = M.tm[k];
-    int vol, u, v0;
-    coords(k, t, vol, u, v0);
+    int vol, u, v0, nl;
+    coords(k, t, vol, u, v0, nl);
     mbar_wait_bounded(&full[cur], (it >> 1) & 1, WF_LINE_PASS);
-    if (threadIdx.x == 0 && t + (int)gridDim.x < total) issue(t + gridDim.x, cur ^ 1);
-    // the shear coefficients depend on the job and volume only (the barrier before the
-    // previous tile's store separates every read of coef_s from this write)
-    if (k != coef_job || vol != coef_vol) {
-      if (threadIdx.x == 0) {
-        PhaseCoef cf{0, 0, 0};
-        if (A.params) cf = phase_coef(A.ph[0], A.params + (i64)vol * A.pstride, A.ax);
-        coef_s = cf;
-      }
-      coef_job = k;
-      coef_vol = vol;
-      __syncthreads();
+    if (mover && t + (int)gridDim.x < total) issue(t + gridDim.x, cur ^ 1);
+    if (k != coef_job) coef_vol = -1;
+    coef_job = k;
+    set_coefs<false>(A, vol, coef_vol, coef_s);
+    int ul = u, vl = v0 + min(g, nl - 1);
+    if (!STRIDED) {
+      const int l = u * A.dims[A.av] + vl;
+      ul = A.div_av.div(l);
+      vl = l - ul * A.dims[A.av];
     }
-    const bool id0 = phase_is_identity(A.ph[0]);
-    int c[3];
-    c[A.au] = u;
-    c[A.av] = v0 + g;
-    c[A.ax] = 0;
-    const bool sep0 = !id0 && A.ph[0].sep;
-    const PhaseCoef c0 = coef_s;
-    Ch ch0;
-    if (sep0) ch0.init(A.ph[0], c0, A.ph[0].rvec ? A.ph[0].rvec[c[A.ph[0].oaxis]] : 0.0, j, A.scale, A.scale_lo, G);
     unsigned char* tb = tiles + cur * TILE;
-    float2* L = scratch + g * LS;
-    float2 X[R2];
-    F::forward_from([&](int n) { return *reinterpret_cast<const float2*>(tb + tile_off<N, B, STRIDED>(g, n)); },
-                    L, j, X);
-    if (j < R1) {
-      if (id0) {
-#pragma unroll
-        for (int r = 0; r < R2; r++) X[r] = cscale2(X[r], A.scale, A.scale_lo);
-      } else if (sep0) {
-        ch0.apply(X);
-      } else {
-#pragma unroll
-        for (int r = 0; r < R2; r++) {
-          c[A.ax] = j + r * R1;
-          X[r] = cmul(X[r], phase_value(A.ph[0], c0, j + r * R1, c, A.scale, A.scale_lo));
-        }
-      }
-    }
-    F::inverse_to(L, j, X, [&](int, int n, float2 v) {
-      *reinterpret_cast<float2*>(tb + tile_off<N, B, STRIDED>(g, n)) = v;
-    });
+    s0.line = tb + (STRIDED ? 0 : g * PITCH);
+    pass_line<N, PM_SHEAR>(A, coef_s, ul, vl, j, s0, s0, chirp_s[g]);
     fence_proxy_async_smem();
     __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll
-      for (int q = 0; q < NSUB; q++) {
-        const unsigned char* src = tb + q * SUBT;
-        const int c0s = STRIDED ? v0 + 16 * q : 0, c1s = STRIDED ? 0 : v0;
-        if (J.out_rank == 3) {
-          tma_store_3d(&J.out, src, c0s, c1s, u);
-        } else {
-          tma_store_4d(&J.out, src, c0s, c1s, u, vol);
+    if (mover) {
+      if (STRIDED) {
+        if (threadIdx.x == 0) {
+          if (J.out_rank == 3) tma_store_3d(&J.out, tb, v0, 0, u);
+          else tma_store_4d(&J.out, tb, v0, 0, u, vol);
         }
+      } else if ((int)threadIdx.x < nl) {
+        bulk_s2g(A.out0 + (i64)vol * A.out_vs + tile_line(A, u, v0, threadIdx.x),
+                 tb + threadIdx.x * PITCH, N * 8);
       }
       bulk_commit();
     }
   }
-  if (threadIdx.x == 0) bulk_wait_all();
+  if (mover) bulk_wait_all();
 }
 
-template <int N, int R1, int R2, bool STRIDED>
-static int launch_tma_multi_n(const MultiTmaArgs& M, cudaStream_t stream) {
-  using F = LineFft<N, R1, R2>;
-  constexpr int B = 256 / F::G;
-  const size_t smem = 1024 + 2 * (size_t)B * N * 8 + sizeof(float2) * (size_t)F::LS * B;
-  auto kern = tma_multi_shear_kernel<N, R1, R2, STRIDED>;
+template <typename K, typename M>
+static int launch_multi_kernel(K kern, const M& args, int threads, size_t smem, cudaStream_t stream) {
   const int rc = check_cuda(allow_smem(kern, smem), "multi shear smem");
   if (rc != ME_OK) return rc;
   int dev = 0, sms = 148, nb = 2;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, 256, smem);
-  const int total = M.tile_off[M.njobs];
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, threads, smem);
+  const int total = args.tile_off[args.njobs];
   const int grid = (int)std::min<long long>(total, (long long)std::max(1, nb) * sms);
   count_launch();
-  kern<<<grid, 256, smem, stream>>>(M);
+  kern<<<grid, threads, smem, stream>>>(args);
   return check_cuda(cudaGetLastError(), "multi shear launch");
 }
 
-template <int N, int R1, int R2>
+template <int N, bool STRIDED>
+static int launch_tma_multi_n(const MultiTmaArgs& M, cudaStream_t stream) {
+  return launch_multi_kernel(tma_multi_shear_kernel<N, STRIDED>, M, PassLine<N>::THREADS,
+                             1024 + 2 * (size_t)TileShape<N, STRIDED>::TILE, stream);
+}
+
+template <int N>
 static int launch_multi_n(const MultiPassArgs& M, cudaStream_t stream) {
-  using F = LineFft<N, R1, R2>;
-  const size_t smem = 2 * sizeof(float2) * (size_t)F::LS * (256 / F::G);
-  const int rc = check_cuda(allow_smem(multi_shear_kernel<N, R1, R2>, smem), "multi shear smem");
-  if (rc != ME_OK) return rc;
-  int dev = 0, sms = 148, nb = 2;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, multi_shear_kernel<N, R1, R2>, 256, smem);
-  const int total = M.tile_off[M.njobs];
-  const int grid = (int)std::min<long long>(total, (long long)std::max(1, nb) * sms);
-  count_launch();
-  multi_shear_kernel<N, R1, R2><<<grid, 256, smem, stream>>>(M);
-  return check_cuda(cudaGetLastError(), "multi shear launch");
+  return launch_multi_kernel(multi_shear_kernel<N>, M, PassLine<N>::THREADS,
+                             2 * (size_t)kTileLines * line_pitch(N), stream);
 }
 
 static bool fast_length(int n) {
@@ -1289,16 +938,6 @@ static bool fast_length(int n) {
     ME_FAST_LENGTHS(ME_FAST_IS)
 #undef ME_FAST_IS
     default: return false;
-  }
-}
-
-static int tile_lines(int n) {
-  switch (n) {
-#define ME_TILE_LINES(N, R1, R2) \
-  case N: return 256 / LineFft<N, R1, R2>::G;
-    ME_FAST_LENGTHS(ME_TILE_LINES)
-#undef ME_TILE_LINES
-    default: return 0;
   }
 }
 
@@ -1316,49 +955,50 @@ int launch_multi_shear(const PassArgs* jobs, int njobs, cudaStream_t stream) {
     if (done[k0]) continue;
     const int n = jobs[k0].plan.n;
     MultiPassArgs M;
+    MultiTmaArgs MT;
     M.njobs = 0;
-    M.tile_off[0] = 0;
-    long long total = 0;
+    // on TMA tiles when every job of this length qualifies
+    bool tma = true, strided = true;
     for (int k = k0; k < njobs; k++) {
       if (done[k] || jobs[k].plan.n != n) continue;
       done[k] = true;
-      const int B = tile_lines(n);
-      total += (long long)((jobs[k].nlines + B - 1) / B) * jobs[k].nvol;
+      const int q = M.njobs++;
+      M.job[q] = jobs[k];
+      PassTma T;
+      bool s = false;
+      tma = tma && tma_pass_setup(PM_SHEAR, jobs[k], &s, &T);
+      if (!tma) continue;
+      if (q == 0) strided = s;
+      tma = (s == strided);
+      MT.tm[q].in = T.in[0];
+      MT.tm[q].out = T.out[0];
+      MT.tm[q].in_rank = T.in_rank[0];
+      MT.tm[q].out_rank = T.out_rank[0];
+      MT.tm[q].div_row = T.div_row;
+      MT.tm[q].row_tiles = T.row_tiles;
+    }
+    long long total = 0;
+    M.tile_off[0] = 0;
+    for (int q = 0; q < M.njobs; q++) {
+      const int tiles = tiles_of(M.job[q], tma && strided);
+      total += (long long)tiles * M.job[q].nvol;
       if (total > 0x7fffffffLL) return fail("multi shear: too many work items");
-      M.job[M.njobs] = jobs[k];
-      M.job[M.njobs].div_tiles.set((jobs[k].nlines + B - 1) / B);
-      M.tile_off[++M.njobs] = (int)total;
+      M.job[q].div_tiles.set(std::max(1, tiles));
+      M.tile_off[q + 1] = (int)total;
     }
     if (total == 0) continue;
-    // on TMA tiles when every job of this length qualifies
-    const int B = tile_lines(n);
-    MultiTmaArgs MT;
-    bool tma = true, all_strided = true;
-    for (int q = 0; q < M.njobs && tma; q++) {
-      PassTma T;
-      bool strided = false;
-      tma = tma_pass_setup(PM_SHEAR, M.job[q], B, &strided, &T);
-      if (tma) {
-        if (q == 0) all_strided = strided;
-        tma = (strided == all_strided);
-        MT.job[q] = M.job[q];
-        MT.tm[q].in = T.in[0];
-        MT.tm[q].out = T.out[0];
-        MT.tm[q].in_rank = T.in_rank[0];
-        MT.tm[q].out_rank = T.out_rank[0];
-      }
-    }
     if (tma) {
       MT.njobs = M.njobs;
+      for (int q = 0; q < M.njobs; q++) MT.job[q] = M.job[q];
       for (int q = 0; q <= M.njobs; q++) MT.tile_off[q] = M.tile_off[q];
     }
     int rc = -1;
     switch (n) {
-#define ME_MULTI_LAUNCH(N, R1, R2)                                                  \
-  case N:                                                                           \
-    rc = !tma ? launch_multi_n<N, R1, R2>(M, stream)                                 \
-         : all_strided ? launch_tma_multi_n<N, R1, R2, true>(MT, stream)            \
-                       : launch_tma_multi_n<N, R1, R2, false>(MT, stream);          \
+#define ME_MULTI_LAUNCH(N, R1, R2)                                             \
+  case N:                                                                      \
+    rc = !tma ? launch_multi_n<N>(M, stream)                               \
+         : strided ? launch_tma_multi_n<N, true>(MT, stream)               \
+                   : launch_tma_multi_n<N, false>(MT, stream);             \
     break;
       ME_FAST_LENGTHS(ME_MULTI_LAUNCH)
 #undef ME_MULTI_LAUNCH

@@ -44,4 +44,15 @@ __device__ __forceinline__ float2 phase_value(const Phase& P, const PhaseCoef& C
   return cscale2(e, scale, scale_lo);
 }
 
+// Phase q of pass A at (u, v) along axes au and av, as a call: for the rare grids whose phases
+// are no line chirps.
+__device__ __noinline__ static float2 phase_value_call(const PassArgs& A, int q, PhaseCoef C,
+                                                       int n, int u, int v) {
+  int c[3];
+  c[A.au] = u;
+  c[A.av] = v;
+  c[A.ax] = n;
+  return phase_value(A.ph[q], C, n, c, A.scale, A.scale_lo);
+}
+
 }  // namespace me

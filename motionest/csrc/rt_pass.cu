@@ -34,15 +34,18 @@ static double radix_gain(int r) {
   return radix_gain(a) * radix_gain(r / a) * twiddle_gain(r, a, r / a);
 }
 
-double fft_pair_gain(int n) {
-  static std::atomic<double> known[ME_MAX_LINE + 1];
+static double plan_gain(int n, bool sense) {
+  static std::atomic<double> known[2][ME_MAX_LINE + 1];
   if (n < 1 || n > ME_MAX_LINE) return 1.0;
-  double g = known[n].load(std::memory_order_relaxed);
+  double g = known[sense][n].load(std::memory_order_relaxed);
   if (g != 0.0) return g;
   int r1 = 0, r2 = 0;
   switch (n) {
-#define ME_GAIN_CASE(N, R1, R2) \
-  case N: r1 = R1; r2 = R2; break;
+#define ME_GAIN_CASE(N, R1, R2)     \
+  case N:                           \
+    r2 = sense ? R2 : N <= 128 ? 8 : 16; \
+    r1 = N / r2;                    \
+    break;
     ME_FAST_LENGTHS(ME_GAIN_CASE)
 #undef ME_GAIN_CASE
     default: {
@@ -54,9 +57,12 @@ double fft_pair_gain(int n) {
     }
   }
   g = r1 ? radix_gain(r1) * radix_gain(r2) * twiddle_gain(n, r1, r2) : 1.0;
-  known[n].store(g, std::memory_order_relaxed);
+  known[sense][n].store(g, std::memory_order_relaxed);
   return g;
 }
+
+double fft_pair_gain(int n) { return plan_gain(n, false); }
+double sense_fft_pair_gain(int n) { return plan_gain(n, true); }
 
 int try_rt_pass(int mode, PassArgs& A, cudaStream_t stream) {
   RtPlan P;

@@ -1047,7 +1047,7 @@ static bool fast_sense_enabled() {
 
 // 1/sqrt(XY), with the gain of the FFT along y taken out
 static double sense_scale(const me_sense* pb) {
-  return 1.0 / sqrt((double)pb->nx * pb->ny * (fast_sense_enabled() ? fft_pair_gain(pb->ny) : 1.0));
+  return 1.0 / sqrt((double)pb->nx * pb->ny * (fast_sense_enabled() ? sense_fft_pair_gain(pb->ny) : 1.0));
 }
 
 static int fwd_rows(int V, int Y) {
