@@ -1,16 +1,21 @@
 // Register-resident small DFTs and the two-stage line FFT used by the compile-time kernels.
 //
-// A line of length N = R1 * R2 is owned by a group of G threads (G = 16 or 8, inside one
-// warp) and lives in a shared-memory region of LS elements.  Forward transform:
-//   stage 1: thread j < R2 reads x[j + r R2] (r < R1), does an R1-point DFT in registers and
-//            writes Y_j[k] to row j of a padded [R2][S1] table (S1 = R1 rounded up to odd);
-//   stage 2: thread j < R1 reads column j (Y_r[j], r < R2), multiplies by W_N^{r j} (from a
-//            table in that order), does an R2-point DFT and ends holding X[j + r R1] for
-//            r < R2 in registers.
-// The inverse transform consumes that register layout directly (inverse R2-point DFT,
-// W_N^{-j a}, transpose through the padded table, inverse R1-point DFT) and writes x in natural
-// order.  Only __syncwarp is needed between the steps, all index arithmetic is compile-time,
-// and every shared-memory access pattern is bank-conflict free (unit or odd strides).
+// A line of N = G R1 points belongs to G threads (G = 8 up to 128 points, 16 above) and N slots of
+// shared memory:
+//   stage 1: thread j < G transforms x[j + G r], r < R1, in registers and puts output k into slot
+//            G k + (j + k) mod G;
+//   stage 2: item k (thread k mod G, up to two items each) reads row k, multiplies by W_N^{r k}
+//            and transforms its G points into X[k + R1 r].
+// The inverse runs the same steps backwards.
+//
+// Why the second radix is the number of threads: no lane idles in the first stage and few do in
+// the second (R1 of G ceil(R1/G) items).  With plans that led with a 16-point stage, 9 of 16 lanes
+// idled in it at 112 = 16 x 7 points (133 instructions per voxel of a line pass; 128 = 16 x 8: 119).
+// The lanes are dealt so that a half warp holds eight threads of each of two neighbouring lines:
+// with a row's start turned by k these touch 16 distinct 8-byte banks in every access, in a tile
+// that interleaves the two lines or keeps them 64 bytes apart modulo 128, and the transposes need
+// no scratch beside the line.  Only __syncwarp separates the stages, and all index arithmetic but
+// the turns is compile-time.
 #pragma once
 #include "common.cuh"
 #include "dft_consts.cuh"
@@ -100,6 +105,14 @@ template <bool INV> struct RDft<7, INV> : RDftPrime<7, INV> {};
 template <bool INV> struct RDft<11, INV> : RDftPrime<11, INV> {};
 template <bool INV> struct RDft<13, INV> : RDftPrime<13, INV> {};
 
+// t *= W_R^m for a compile-time m, quarter turns without a multiplication.
+template <int R, bool INV>
+__device__ __forceinline__ float2 mul_wr(float2 t, int m) {
+  if (m == 0) return t;
+  if (4 * m == R) return INV ? mul_i(t) : mul_mi(t);
+  return cmul(t, wr<R, INV>(m));
+}
+
 // Composite R = A * B: n = B n1 + n2, k = k1 + A k2,
 // X[k1 + A k2] = sum_{n2} W_R^{n2 k1} W_B^{n2 k2} sum_{n1} x[B n1 + n2] W_A^{n1 k1}.
 template <int A, int B, bool INV>
@@ -114,8 +127,7 @@ struct RDftComp {
       for (int n1 = 0; n1 < A; n1++) u[n1] = v[B * n1 + n2];
       RDft<A, INV>::run(u);
 #pragma unroll
-      for (int k1 = 0; k1 < A; k1++)
-        t[n2 * A + k1] = (n2 * k1 == 0) ? u[k1] : cmul(u[k1], wr<R, INV>(n2 * k1));
+      for (int k1 = 0; k1 < A; k1++) t[n2 * A + k1] = mul_wr<R, INV>(u[k1], n2 * k1);
     }
 #pragma unroll
     for (int k1 = 0; k1 < A; k1++) {
@@ -129,129 +141,220 @@ struct RDftComp {
   }
 };
 
-template <bool INV> struct RDft<6, INV> : RDftComp<2, 3, INV> {};
+// Coprime R = A * B by the prime-factor map (Good, 1958): n = B n1 + A n2 and k = k1 mod A,
+// k2 mod B turn the DFT into A- and B-point DFTs with no twiddles between (14 points: 156
+// floating-point instructions instead of 184).
+template <int A, int B, bool INV>
+struct RDftPfa {
+  // the multiple of B that is 1 mod A (E1) and the multiple of A that is 1 mod B (E2)
+  static constexpr int unit(int mult, int mod) {
+    int e = mult;
+    while (e % mod != 1) e += mult;
+    return e;
+  }
+  static __device__ __forceinline__ void run(float2* v) {
+    constexpr int R = A * B, E1 = unit(B, A), E2 = unit(A, B);
+    float2 t[R];
+#pragma unroll
+    for (int n2 = 0; n2 < B; n2++) {
+      float2 u[A];
+#pragma unroll
+      for (int n1 = 0; n1 < A; n1++) u[n1] = v[(B * n1 + A * n2) % R];
+      RDft<A, INV>::run(u);
+#pragma unroll
+      for (int k1 = 0; k1 < A; k1++) t[n2 * A + k1] = u[k1];
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < A; k1++) {
+      float2 w[B];
+#pragma unroll
+      for (int n2 = 0; n2 < B; n2++) w[n2] = t[n2 * A + k1];
+      RDft<B, INV>::run(w);
+#pragma unroll
+      for (int k2 = 0; k2 < B; k2++) v[(E1 * k1 + E2 * k2) % R] = w[k2];
+    }
+  }
+};
+
+template <bool INV> struct RDft<6, INV> : RDftPfa<2, 3, INV> {};
+template <bool INV> struct RDft<10, INV> : RDftPfa<2, 5, INV> {};
+template <bool INV> struct RDft<12, INV> : RDftPfa<4, 3, INV> {};
+template <bool INV> struct RDft<14, INV> : RDftPfa<2, 7, INV> {};
+template <bool INV> struct RDft<15, INV> : RDftPfa<3, 5, INV> {};
+template <bool INV> struct RDft<18, INV> : RDftPfa<2, 9, INV> {};
+template <bool INV> struct RDft<20, INV> : RDftPfa<4, 5, INV> {};
+template <bool INV> struct RDft<21, INV> : RDftPfa<3, 7, INV> {};
+template <bool INV> struct RDft<22, INV> : RDftPfa<2, 11, INV> {};
+template <bool INV> struct RDft<24, INV> : RDftPfa<8, 3, INV> {};
+template <bool INV> struct RDft<26, INV> : RDftPfa<2, 13, INV> {};
+template <bool INV> struct RDft<28, INV> : RDftPfa<4, 7, INV> {};
+template <bool INV> struct RDft<30, INV> : RDftPfa<2, 15, INV> {};
 template <bool INV> struct RDft<8, INV> : RDftComp<2, 4, INV> {};
 template <bool INV> struct RDft<9, INV> : RDftComp<3, 3, INV> {};
-template <bool INV> struct RDft<12, INV> : RDftComp<4, 3, INV> {};
-template <bool INV> struct RDft<14, INV> : RDftComp<2, 7, INV> {};
 template <bool INV> struct RDft<16, INV> : RDftComp<4, 4, INV> {};
-// radices of the run-time plans only (fft_rt.cuh)
-template <bool INV> struct RDft<10, INV> : RDftComp<2, 5, INV> {};
-template <bool INV> struct RDft<15, INV> : RDftComp<3, 5, INV> {};
-template <bool INV> struct RDft<18, INV> : RDftComp<2, 9, INV> {};
-template <bool INV> struct RDft<20, INV> : RDftComp<4, 5, INV> {};
-template <bool INV> struct RDft<21, INV> : RDftComp<3, 7, INV> {};
-template <bool INV> struct RDft<22, INV> : RDftComp<2, 11, INV> {};
-template <bool INV> struct RDft<24, INV> : RDftComp<4, 6, INV> {};
 template <bool INV> struct RDft<25, INV> : RDftComp<5, 5, INV> {};
-template <bool INV> struct RDft<26, INV> : RDftComp<2, 13, INV> {};
 template <bool INV> struct RDft<27, INV> : RDftComp<3, 9, INV> {};
-template <bool INV> struct RDft<28, INV> : RDftComp<4, 7, INV> {};
-template <bool INV> struct RDft<30, INV> : RDftComp<5, 6, INV> {};
 template <bool INV> struct RDft<32, INV> : RDftComp<4, 8, INV> {};
 
-// Second-stage twiddle W_N^{r j} from the plan-ordered table: for each r the R1 threads of a
-// line read R1 consecutive entries (one L1 wavefront per warp instead of one sector per
-// thread, as indices r j mod N scattered over the natural-order table would need).
+// Second-stage twiddles W_N^{r k} in the order r R1 + k.
 template <int N> __device__ __forceinline__ const float2* twp_table();
-#define ME_TWP_TABLE(N, R1, R2) \
+#define ME_TWP_TABLE(N) \
   template <> __device__ __forceinline__ const float2* twp_table<N>() { return twp##N; }
 ME_FAST_LENGTHS(ME_TWP_TABLE)
 #undef ME_TWP_TABLE
 
-template <int N, int R1, bool INV>
-__device__ __forceinline__ float2 twP(int r, int j) {
-  float2 w = __ldg(twp_table<N>() + r * R1 + j);
-  if (INV) w.y = -w.y;
-  return w;
+__host__ __device__ constexpr int line_threads(int n) { return n <= 128 ? 8 : 16; }
+
+// Bytes between the lines of a linear tile: a multiple of 16, 64 modulo 128.
+__host__ __device__ constexpr int line_pitch(int n) { return n * 8 + (n % 16 == 0 ? 64 : 0); }
+
+// This thread's line g of the CTA's and its place j < G in it.
+template <int G>
+__device__ __forceinline__ void line_place(int& g, int& j) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (G == 8) {
+    g = warp * 4 + (lane >> 3);
+    j = lane & 7;
+  } else {
+    g = warp * 2 + ((lane >> 3) & 1);
+    j = (lane & 7) | ((lane >> 4) << 3);
+  }
 }
 
-template <int N, int R1, int R2>
+// A line's slots in a tile, as thread j of the line sees them.  A row of G slots is ROW bytes from
+// the next; slot (j + q) mod G of a row lies at F[q mod 8], the other half of 16 slots at XOR HALF.
+//   STRIDED: tile [n][16 lines] with the tensor map's 128-byte swizzle (the 16-byte chunk of
+//     line pair g / 2 at index n is g / 2 XOR n mod 8);
+//   else: the line's N slots in a row, neighbouring lines 64 bytes apart modulo 128.
+template <int G, bool STRIDED>
+struct Slots {
+  static constexpr int ROW = STRIDED ? 128 * G : 8 * G;
+  static constexpr int HALF = STRIDED ? 1024 : 64;
+  unsigned char* line;
+  int F[8];
+  int g;
+  __device__ __forceinline__ int in_row(int m) const {
+    return STRIDED ? m * 128 + ((((g >> 1) ^ m) & 7) << 4) + ((g & 1) << 3) : m * 8;
+  }
+  __device__ __forceinline__ void init(int g_, int j) {
+    g = g_;
+#pragma unroll
+    for (int q = 0; q < 8; q++) F[q] = in_row((j + q) & (G - 1));
+  }
+  // row `row`, slot (j + q) mod G
+  __device__ __forceinline__ float2& tab(int row, int q) const {
+    const int f = F[q & 7] ^ ((G == 16 && (q & 8)) ? HALF : 0);
+    return *reinterpret_cast<float2*>(line + f + row * ROW);
+  }
+  __device__ __forceinline__ float2& at(int n) const {
+    return *reinterpret_cast<float2*>(line + (n / G) * ROW + in_row(n & (G - 1)));
+  }
+  __device__ __forceinline__ float2& put(int k) const { return tab(k, k); }
+  __device__ __forceinline__ float2& row(int k, int r) const { return tab(k, r); }
+};
+
+// Slots of a line that has a region of its own beside the data (line_region elements): rows by
+// thread with an odd stride, so that all offsets but the thread's own are compile-time.  Free of
+// bank conflicts with sixteen threads of one line to a half warp, and with eight of two lines
+// whose regions lie 8 elements apart modulo 16.
+__host__ __device__ constexpr int line_region(int n) {
+  const int g = line_threads(n), r1 = n / g, need = g * (r1 | 1) > n ? g * (r1 | 1) : n;
+  return (need + 7) / 16 * 16 + 8;
+}
+template <int N>
+struct PaddedSlots {
+  static constexpr int S1 = (N / line_threads(N)) | 1;
+  float2* line;
+  float2* mine;  // line + j S1
+  __device__ __forceinline__ void init(float2* l, int j) {
+    line = l;
+    mine = l + j * S1;
+  }
+  __device__ __forceinline__ float2& at(int n) const { return line[n]; }
+  __device__ __forceinline__ float2& put(int k) const { return mine[k]; }
+  __device__ __forceinline__ float2& row(int k, int r) const { return line[r * S1 + k]; }
+};
+
+template <int N>
 struct LineFft {
-  static constexpr int S1 = R1 | 1;  // odd row stride of the transpose table
-  static constexpr int LS = ((N > R2 * S1 ? N : R2 * S1)) | 1;
-  static constexpr int G = (R1 > R2 ? R1 : R2) <= 8 ? 8 : 16;
+  static constexpr int G = line_threads(N);
+  static constexpr int R1 = N / G;
+  static constexpr int NI = (R1 + G - 1) / G;  // stage 2 items per thread
 
-  // Forward FFT of the natural-order line in L; thread j (< R1) ends with X[j + r R1].
-  static __device__ __forceinline__ void forward(float2* L, int j, float2 (&X)[R2]) {
-    forward_from([&](int n) { return L[n]; }, L, j, X);
-  }
-
-  // Forward FFT of the line x[n] = load(n) (read once, in the first stage); L is the line's
-  // work region and may differ from where load() reads.
-  template <class Load>
-  static __device__ __forceinline__ void forward_from(Load load, float2* L, int j, float2 (&X)[R2]) {
+  // Stage 1 of x[n] = load(r, n) (n = j + G r, read once) into the turned slots.  IN_PLACE: load
+  // reads the slots themselves, which other threads are about to overwrite.
+  template <bool IN_PLACE, class S, class Load>
+  static __device__ __forceinline__ void first(const S& s, int j, Load load) {
     float2 u[R1];
-    if (j < R2) {
 #pragma unroll
-      for (int r = 0; r < R1; r++) u[r] = load(j + r * R2);
-      RDft<R1, false>::run(u);
-    }
+    for (int r = 0; r < R1; r++) u[r] = load(r, j + G * r);
+    RDft<R1, false>::run(u);
+    if (IN_PLACE) __syncwarp();
+#pragma unroll
+    for (int k = 0; k < R1; k++) s.put(k) = u[k];
     __syncwarp();
-    if (j < R2) {
+  }
+  // Stage 3: the turned slots to store(r, n, x[n]).
+  template <bool IN_PLACE, class S, class Store>
+  static __device__ __forceinline__ void last(const S& s, int j, Store store) {
+    float2 u[R1];
 #pragma unroll
-      for (int r = 0; r < R1; r++) L[j * S1 + r] = u[r];
+    for (int k = 0; k < R1; k++) u[k] = s.put(k);
+    RDft<R1, true>::run(u);
+    if (IN_PLACE) __syncwarp();
+#pragma unroll
+    for (int r = 0; r < R1; r++) store(r, j + G * r, u[r]);
+  }
+  // Row k = j + G i to its spectrum X[k + R1 r] and back.
+  template <class S>
+  static __device__ __forceinline__ void row_forward(const S& s, int k, float2 (&X)[G]) {
+#pragma unroll
+    for (int r = 0; r < G; r++) {
+      const float2 y = s.row(k, r);
+      X[r] = (r == 0) ? y : cmul(y, __ldg(twp_table<N>() + r * R1 + k));
     }
-    __syncwarp();
-    if (j < R1) {
+    RDft<G, false>::run(X);
+  }
+  template <class S>
+  static __device__ __forceinline__ void row_inverse(const S& s, int k, float2 (&X)[G]) {
+    RDft<G, true>::run(X);
 #pragma unroll
-      for (int r = 0; r < R2; r++) {
-        const float2 y = L[r * S1 + j];
-        X[r] = (r == 0) ? y : cmul(y, twP<N, R1, false>(r, j));
+    for (int r = 0; r < G; r++)
+      s.row(k, r) = (r == 0) ? X[r] : cmulc(X[r], __ldg(twp_table<N>() + r * R1 + k));
+  }
+  // Forward transform of load(r, n) to the natural-order spectrum in the line's slots, and the
+  // inverse of that spectrum to store(r, n, x[n]).  The natural slots of one row's results belong
+  // to other rows, so a thread holds all its rows before any is written.
+  template <class S, class Load>
+  static __device__ __forceinline__ void forward(const S& s, int j, Load load) {
+    first<false>(s, j, load);
+    float2 X[NI][G];
+#pragma unroll
+    for (int i = 0; i < NI; i++)
+      if (R1 % G == 0 || j + G * i < R1) row_forward(s, j + G * i, X[i]);
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < NI; i++)
+      if (R1 % G == 0 || j + G * i < R1) {
+#pragma unroll
+        for (int r = 0; r < G; r++) s.at(j + G * i + R1 * r) = X[i][r];
       }
-      RDft<R2, false>::run(X);
-    }
   }
-
-  // Inverse FFT from the register layout of forward(); writes x in natural order into L.
-  static __device__ __forceinline__ void inverse(float2* L, int j, float2 (&X)[R2]) {
-    inverse_to(L, j, X, [&](int b, int n, float2 v) { L[n] = v; });
-    __syncwarp();
-  }
-
-  // Inverse FFT handing each output to store(b, n, x[n]) (b < R1 the compile-time slot, n = j +
-  // b R2, threads j < R2) instead of writing it to L; L is the line's work region.
-  template <class Store>
-  static __device__ __forceinline__ void inverse_to(float2* L, int j, float2 (&X)[R2], Store store) {
-    if (j < R1) {
-      RDft<R2, true>::run(X);
+  template <class S, class Store>
+  static __device__ __forceinline__ void inverse(const S& s, int j, Store store) {
+    float2 X[NI][G];
 #pragma unroll
-      for (int a = 1; a < R2; a++) X[a] = cmul(X[a], twP<N, R1, true>(a, j));
-    }
-    __syncwarp();
-    if (j < R1) {
+    for (int i = 0; i < NI; i++)
+      if (R1 % G == 0 || j + G * i < R1) {
 #pragma unroll
-      for (int a = 0; a < R2; a++) L[a * S1 + j] = X[a];
-    }
+        for (int r = 0; r < G; r++) X[i][r] = s.at(j + G * i + R1 * r);
+      }
     __syncwarp();
-    float2 u[R1];
-    if (j < R2) {
 #pragma unroll
-      for (int b = 0; b < R1; b++) u[b] = L[j * S1 + b];
-      RDft<R1, true>::run(u);
-    }
+    for (int i = 0; i < NI; i++)
+      if (R1 % G == 0 || j + G * i < R1) row_inverse(s, j + G * i, X[i]);
     __syncwarp();
-    if (j < R2) {
-#pragma unroll
-      for (int b = 0; b < R1; b++) store(b, j + b * R2, u[b]);
-    }
-  }
-
-  // Natural-order spectrum from registers (thread j holds X[j + r R1]).
-  static __device__ __forceinline__ void store_spectrum(float2* L, int j, const float2 (&X)[R2]) {
-    __syncwarp();
-    if (j < R1) {
-#pragma unroll
-      for (int r = 0; r < R2; r++) L[j + r * R1] = X[r];
-    }
-    __syncwarp();
-  }
-
-  static __device__ __forceinline__ void load_spectrum(const float2* L, int j, float2 (&X)[R2]) {
-    if (j < R1) {
-#pragma unroll
-      for (int r = 0; r < R2; r++) X[r] = L[j + r * R1];
-    }
+    last<false>(s, j, store);
   }
 };
 

@@ -45,7 +45,8 @@ inline double rt_radix_cost(int r) {
     if (r == p[i]) break;
     if (r % p[i] == 0) {
       const int a = p[i], b = r / p[i];
-      return rt_radix_cost(a) + rt_radix_cost(b) + 4.0 * (a - 1) * (b - 1) / r;
+      const bool coprime = (a % 2 || b % 2) && (a % 3 || b % 3) && (a % 5 || b % 5);
+      return rt_radix_cost(a) + rt_radix_cost(b) + (coprime ? 0.0 : 4.0 * (a - 1) * (b - 1) / r);
     }
   }
   if (r == 2) return 2.0;

@@ -15,12 +15,8 @@ import numpy as np
 HERE = Path(__file__).resolve().parent
 OUT = HERE / "dft_consts.cuh"
 
-# Line lengths with a compile-time two-stage plan N = R1 * R2 (R1, R2 <= 16).
-PLANS = {
-    16: (4, 4), 24: (8, 3), 32: (8, 4), 48: (16, 3), 56: (8, 7), 64: (8, 8), 72: (8, 9),
-    88: (8, 11), 96: (16, 6), 112: (16, 7), 128: (16, 8), 144: (16, 9), 176: (16, 11),
-    192: (16, 12), 224: (16, 14), 256: (16, 16),
-}
+# Line lengths with a compile-time two-stage plan N = G * R1, G = 8 up to 128 points, else 16.
+LENGTHS = [16, 24, 32, 48, 56, 64, 72, 88, 96, 112, 128, 144, 176, 192, 224, 256]
 RADICES = [2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 18, 20, 21, 22, 24, 25, 26, 27,
            28, 30, 32]
 
@@ -35,33 +31,23 @@ def f32(v):
 def main():
     lines = ["// Generated by gen_twiddles.py -- do not edit.", "#pragma once", "",
              "namespace me {", ""]
-    lines.append("// Two-stage plans N = R1 * R2 for the compile-time line FFTs.")
+    lines.append("// Lengths with a compile-time plan (LineFft, fft_reg.cuh).")
     lines.append("#define ME_FAST_LENGTHS(X) \\")
-    items = [f"  X({n}, {r1}, {r2})" for n, (r1, r2) in sorted(PLANS.items())]
-    lines.append(" \\\n".join(items))
+    lines.append(" \\\n".join(f"  X({n})" for n in LENGTHS))
     lines.append("")
-    for n in sorted(PLANS):
+    for n in LENGTHS:
         m = np.arange(n)
         ang = -2.0 * np.pi * m / n
         vals = ", ".join(f"{{{f32(np.cos(a))}, {f32(np.sin(a))}}}" for a in ang)
         lines.append(f"__device__ const float2 tw{n}[{n}] = {{{vals}}};")
     lines.append("")
     lines.append("// The second-stage twiddles of each plan in the order the threads read them:")
-    lines.append("// twp<N>[r R1 + j] = tw<N>[(r j) mod N] (the same float32 values), so that the R1")
-    lines.append("// threads of a line read R1 consecutive entries for each r.")
-    for n, (r1, r2) in sorted(PLANS.items()):
-        ms = [(r * j) % n for r in range(r2) for j in range(r1)]
-        ang = [-2.0 * np.pi * m / n for m in ms]
-        vals = ", ".join(f"{{{f32(np.cos(a))}, {f32(np.sin(a))}}}" for a in ang)
-        lines.append(f"__device__ const float2 twp{n}[{r1 * r2}] = {{{vals}}};")
-    lines.append("")
-    lines.append("// The twiddles of the line passes' plans N = G R1, G = 8 up to 128 points, else 16")
-    lines.append("// (pass_line.cuh): tp_<N>[r R1 + k] = exp(-2 pi i r k / N), r < G, k < R1.")
-    for n in sorted(PLANS):
+    lines.append("// twp<N>[r R1 + k] = exp(-2 pi i r k / N), r < G, k < R1 = N / G.")
+    for n in LENGTHS:
         g = 8 if n <= 128 else 16
         ang = [-2.0 * np.pi * (r * k) / n for r in range(g) for k in range(n // g)]
         vals = ", ".join(f"{{{f32(np.cos(a))}, {f32(np.sin(a))}}}" for a in ang)
-        lines.append(f"__device__ const float2 tp_{n}[{n}] = {{{vals}}};")
+        lines.append(f"__device__ const float2 twp{n}[{n}] = {{{vals}}};")
     lines.append("")
     lines.append("// cos / sin of 2 pi m / R for the register DFTs (m is a compile-time constant at")
     lines.append("// every call site after unrolling, so these fold to immediates)")

@@ -170,8 +170,7 @@ __global__ void __launch_bounds__(256) line_pass_kernel(const PassArgs A) {
 // CTAs per SM it is compiled for: 16 warps of 128 registers, 20 of 96 at the shortest lengths.
 constexpr int pass_min_ctas(int n, bool dual) { return n > 128 ? 2 : (dual || n > 64) ? 4 : 5; }
 
-// Bytes between the lines of a linear tile: 16-byte multiples, 64 modulo 128.
-constexpr int line_pitch(int n) { return n * 8 + (n % 16 == 0 ? 64 : 0); }
+constexpr int pass_threads(int n) { return kTileLines * line_threads(n); }
 
 // Coefficients of volume `vol`'s phases into shared memory when the CTA moves to another volume
 // (uniform over the CTA, so the barrier is too); their last readers are past a barrier.
@@ -190,10 +189,10 @@ __device__ __forceinline__ void set_coefs(const PassArgs& A, int vol, int& coef_
 
 // Tile staging by cp.async: any strides and alignments, and the plain FFT modes.
 template <int N, int MODE>
-__global__ void __launch_bounds__(PassLine<N>::THREADS,
+__global__ void __launch_bounds__(pass_threads(N),
                                   pass_min_ctas(N, MODE == PM_DUAL_IN || MODE == PM_DUAL_OUT))
     fast_pass_kernel(const __grid_constant__ PassArgs A) {
-  constexpr int G = PassLine<N>::G, B = kTileLines;
+  constexpr int G = LineFft<N>::G, B = kTileLines;
   constexpr bool kDual = (MODE == PM_DUAL_IN || MODE == PM_DUAL_OUT);
   constexpr int NT = kDual ? 2 : 1;    // tiles per buffer
   constexpr int NBUF = kDual ? 1 : 2;
@@ -327,9 +326,9 @@ struct TileShape {
 };
 
 template <int N, int MODE, bool STRIDED>
-__global__ void __launch_bounds__(PassLine<N>::THREADS, pass_min_ctas(N, MODE != PM_SHEAR))
+__global__ void __launch_bounds__(pass_threads(N), pass_min_ctas(N, MODE != PM_SHEAR))
     tma_pass_kernel(const __grid_constant__ PassArgs A, const __grid_constant__ PassTma T) {
-  constexpr int G = PassLine<N>::G;
+  constexpr int G = LineFft<N>::G;
   constexpr bool kDual = (MODE != PM_SHEAR);
   constexpr int NT = kDual ? 2 : 1;  // tiles per buffer
   constexpr int NBUF = kDual ? 1 : 2;
@@ -541,9 +540,9 @@ static int launch_tma(PassArgs& A, const PassTma& T, cudaStream_t stream) {
   const int rc = check_cuda(allow_smem(kern, smem), "tma pass smem");
   if (rc != ME_OK) return rc;
   static std::atomic<int> occ[8];
-  const int grid = pass_grid(kern, PassLine<N>::THREADS, smem, (long long)tiles * A.nvol, occ);
+  const int grid = pass_grid(kern, pass_threads(N), smem, (long long)tiles * A.nvol, occ);
   count_launch();
-  kern<<<grid, PassLine<N>::THREADS, smem, stream>>>(A, T);
+  kern<<<grid, pass_threads(N), smem, stream>>>(A, T);
   return check_cuda(cudaGetLastError(), "tma pass launch");
 }
 
@@ -563,9 +562,9 @@ static int launch_fast(PassArgs& A, cudaStream_t stream) {
   const int rc = check_cuda(allow_smem(kern, smem), "pass smem");
   if (rc != ME_OK) return rc;
   static std::atomic<int> occ[8];
-  const int grid = pass_grid(kern, PassLine<N>::THREADS, smem, (long long)tiles * A.nvol, occ);
+  const int grid = pass_grid(kern, pass_threads(N), smem, (long long)tiles * A.nvol, occ);
   count_launch();
-  kern<<<grid, PassLine<N>::THREADS, smem, stream>>>(A);
+  kern<<<grid, pass_threads(N), smem, stream>>>(A);
   return check_cuda(cudaGetLastError(), "fast pass launch");
 }
 
@@ -583,7 +582,7 @@ static int launch_fast_mode(int mode, PassArgs& A, cudaStream_t stream) {
 // Returns ME_OK / error if handled by a compile-time kernel, -1 if N has no such kernel.
 static int try_fast(int mode, PassArgs& A, cudaStream_t stream) {
   switch (A.plan.n) {
-#define ME_FAST_CASE(N, R1, R2) \
+#define ME_FAST_CASE(N) \
   case N: return launch_fast_mode<N>(mode, A, stream);
     ME_FAST_LENGTHS(ME_FAST_CASE)
 #undef ME_FAST_CASE
@@ -705,9 +704,9 @@ struct MultiPassArgs {
 };
 
 template <int N>
-__global__ void __launch_bounds__(PassLine<N>::THREADS, pass_min_ctas(N, false))
+__global__ void __launch_bounds__(pass_threads(N), pass_min_ctas(N, false))
     multi_shear_kernel(const __grid_constant__ MultiPassArgs M) {
-  constexpr int G = PassLine<N>::G, B = kTileLines;
+  constexpr int G = LineFft<N>::G, B = kTileLines;
   constexpr int PITCH = line_pitch(N), TILE = B * PITCH;
   extern __shared__ __align__(128) unsigned char tiles[];
   __shared__ PhaseCoef coef_s[2];
@@ -804,9 +803,9 @@ struct MultiTmaArgs {
 };
 
 template <int N, bool STRIDED>
-__global__ void __launch_bounds__(PassLine<N>::THREADS, pass_min_ctas(N, false))
+__global__ void __launch_bounds__(pass_threads(N), pass_min_ctas(N, false))
     tma_multi_shear_kernel(const __grid_constant__ MultiTmaArgs M) {
-  constexpr int G = PassLine<N>::G;
+  constexpr int G = LineFft<N>::G;
   constexpr int PITCH = TileShape<N, STRIDED>::PITCH, TILE = TileShape<N, STRIDED>::TILE;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char* tiles = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -921,19 +920,19 @@ static int launch_multi_kernel(K kern, const M& args, int threads, size_t smem, 
 
 template <int N, bool STRIDED>
 static int launch_tma_multi_n(const MultiTmaArgs& M, cudaStream_t stream) {
-  return launch_multi_kernel(tma_multi_shear_kernel<N, STRIDED>, M, PassLine<N>::THREADS,
+  return launch_multi_kernel(tma_multi_shear_kernel<N, STRIDED>, M, pass_threads(N),
                              1024 + 2 * (size_t)TileShape<N, STRIDED>::TILE, stream);
 }
 
 template <int N>
 static int launch_multi_n(const MultiPassArgs& M, cudaStream_t stream) {
-  return launch_multi_kernel(multi_shear_kernel<N>, M, PassLine<N>::THREADS,
+  return launch_multi_kernel(multi_shear_kernel<N>, M, pass_threads(N),
                              2 * (size_t)kTileLines * line_pitch(N), stream);
 }
 
 static bool fast_length(int n) {
   switch (n) {
-#define ME_FAST_IS(N, R1, R2) \
+#define ME_FAST_IS(N) \
   case N: return true;
     ME_FAST_LENGTHS(ME_FAST_IS)
 #undef ME_FAST_IS
@@ -994,7 +993,7 @@ int launch_multi_shear(const PassArgs* jobs, int njobs, cudaStream_t stream) {
     }
     int rc = -1;
     switch (n) {
-#define ME_MULTI_LAUNCH(N, R1, R2)                                             \
+#define ME_MULTI_LAUNCH(N)                                             \
   case N:                                                                      \
     rc = !tma ? launch_multi_n<N>(M, stream)                               \
          : strided ? launch_tma_multi_n<N, true>(MT, stream)               \

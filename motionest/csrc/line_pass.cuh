@@ -82,8 +82,7 @@ int launch_multi_shear(const PassArgs* jobs, int njobs, cudaStream_t stream);
 // Mean gain of a forward and inverse FFT of length n with the float twiddles of its plan
 // (1 - 1e-8 .. 1 - 4e-8, the same for every element and pass, so that twenty passes would add it
 // up); scales divide by it.  1 for a length without a two-stage plan.
-double fft_pair_gain(int n);        // the line passes' plan
-double sense_fft_pair_gain(int n);  // the SENSE kernels' plan
+double fft_pair_gain(int n);
 
 // The pass on the run-time two-stage FFT (rt_pass.cu); -1 when its length has no such plan.
 int try_rt_pass(int mode, PassArgs& A, cudaStream_t stream);

@@ -1,20 +1,6 @@
-// One line of a pass, N = G R1 points by G threads (G = 8 up to 128 points, 16 above): FFT, phase
-// factors, inverse FFT, in place in the line's own N slots of a shared-memory tile.
-//
-//   stage 1: thread j < G transforms x[j + G r], r < R1, in registers and puts output k into slot
-//            G k + (j + k) mod G;
-//   stage 2: item k (thread k mod G, up to two items each) reads row k, multiplies by W_N^{r k},
-//            transforms its G points into X[k + R1 r], multiplies by the phase factors, and runs
-//            the same steps back into the same slots;
-//   stage 3: thread j takes its R1 slots back and writes x[j + G r].
-//
-// Why the second radix is the number of threads: no lane idles in the first stage and few do in
-// the second (R1 of G ceil(R1/G) items).  With plans that led with a 16-point stage, 9 of 16 lanes
-// idled in it at 112 = 16 x 7 points (133 instructions per voxel and pass; 128 = 16 x 8: 119).
-// The lanes are dealt so that a half warp holds eight threads of each of two neighbouring lines:
-// with a row's start turned by k these touch 16 distinct 8-byte banks in every access, in a tile
-// that interleaves the two lines or keeps them 64 bytes apart modulo 128, and the transposes need
-// no scratch beside the tile.  Only __syncwarp separates the stages.
+// One line of a pass by the G threads of its LineFft (fft_reg.cuh): FFT, phase factors, inverse
+// FFT, in place in the line's own N slots of a shared-memory tile.  Between a row's forward and
+// inverse DFT its points get the phase factors, so the spectrum never leaves the registers.
 //
 // The line chirp exp(i C (n - (n >= N/2 ? N : 0))) at n = k + R1 r wraps where r >= G/2, so it is
 // T[r] e_k: the line's T[r], one evaluated by each of its threads into shared memory with the
@@ -27,109 +13,10 @@ namespace me {
 
 constexpr int kTileLines = 16;  // per CTA
 
-__host__ __device__ constexpr int line_threads(int n) { return n <= 128 ? 8 : 16; }
-
-template <int N> __device__ __forceinline__ const float2* tp_table();
-#define ME_TP_TABLE(N, R1, R2) \
-  template <> __device__ __forceinline__ const float2* tp_table<N>() { return tp_##N; }
-ME_FAST_LENGTHS(ME_TP_TABLE)
-#undef ME_TP_TABLE
-
-// This thread's line g of the CTA's 16 and its place j < G in it.
-template <int G>
-__device__ __forceinline__ void line_place(int& g, int& j) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (G == 8) {
-    g = warp * 4 + (lane >> 3);
-    j = lane & 7;
-  } else {
-    g = warp * 2 + ((lane >> 3) & 1);
-    j = (lane & 7) | ((lane >> 4) << 3);
-  }
-}
-
-// A line's slots in a tile, as thread j of the line sees them.  A row of G slots is ROW bytes from
-// the next; slot (j + q) mod G of a row lies at F[q mod 8], the other half of 16 slots at XOR HALF.
-//   STRIDED: tile [n][16 lines] with the tensor map's 128-byte swizzle (the 16-byte chunk of
-//     line pair g / 2 at index n is g / 2 XOR n mod 8);
-//   else: the line's N slots in a row, neighbouring lines 64 bytes apart modulo 128.
-template <int G, bool STRIDED>
-struct Slots {
-  static constexpr int ROW = STRIDED ? 128 * G : 8 * G;
-  static constexpr int HALF = STRIDED ? 1024 : 64;
-  unsigned char* line;
-  int F[8];
-  int g;
-  __device__ __forceinline__ int in_row(int m) const {
-    return STRIDED ? m * 128 + ((((g >> 1) ^ m) & 7) << 4) + ((g & 1) << 3) : m * 8;
-  }
-  __device__ __forceinline__ void init(int g_, int j) {
-    g = g_;
-#pragma unroll
-    for (int q = 0; q < 8; q++) F[q] = in_row((j + q) & (G - 1));
-  }
-  // row `row`, slot (j + q) mod G
-  __device__ __forceinline__ float2& tab(int row, int q) const {
-    const int f = F[q & 7] ^ ((G == 16 && (q & 8)) ? HALF : 0);
-    return *reinterpret_cast<float2*>(line + f + row * ROW);
-  }
-  __device__ __forceinline__ float2& at(int n) const {
-    return *reinterpret_cast<float2*>(line + (n / G) * ROW + in_row(n & (G - 1)));
-  }
-};
-
-template <int N>
-struct PassLine {
-  static constexpr int G = line_threads(N);
-  static constexpr int R1 = N / G;
-  static constexpr int NI = (R1 + G - 1) / G;  // stage 2 items per thread
-  static constexpr int THREADS = kTileLines * G;
-
-  // stages 1 and 3
-  template <class S>
-  static __device__ __forceinline__ void first(const S& s) {
-    float2 u[R1];
-#pragma unroll
-    for (int r = 0; r < R1; r++) u[r] = s.tab(r, 0);
-    RDft<R1, false>::run(u);
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < R1; k++) s.tab(k, k) = u[k];
-    __syncwarp();
-  }
-  template <class S>
-  static __device__ __forceinline__ void last(const S& s) {
-    float2 u[R1];
-#pragma unroll
-    for (int k = 0; k < R1; k++) u[k] = s.tab(k, k);
-    RDft<R1, true>::run(u);
-    __syncwarp();
-#pragma unroll
-    for (int r = 0; r < R1; r++) s.tab(r, 0) = u[r];
-  }
-  // row k = j + G i to its spectrum X[k + R1 r] and back
-  template <class S>
-  static __device__ __forceinline__ void row_forward(const S& s, int k, float2 (&X)[G]) {
-#pragma unroll
-    for (int r = 0; r < G; r++) {
-      const float2 y = s.tab(k, r);
-      X[r] = (r == 0) ? y : cmul(y, __ldg(tp_table<N>() + r * R1 + k));
-    }
-    RDft<G, false>::run(X);
-  }
-  template <class S>
-  static __device__ __forceinline__ void row_inverse(const S& s, int k, float2 (&X)[G]) {
-    RDft<G, true>::run(X);
-#pragma unroll
-    for (int r = 0; r < G; r++)
-      s.tab(k, r) = (r == 0) ? X[r] : cmulc(X[r], __ldg(tp_table<N>() + r * R1 + k));
-  }
-};
-
 // Chirp of one line; T is the line's G table entries in shared memory.
 template <int N>
 struct LineChirp {
-  static constexpr int G = PassLine<N>::G, R1 = PassLine<N>::R1, NI = PassLine<N>::NI;
+  static constexpr int G = LineFft<N>::G, R1 = LineFft<N>::R1, NI = LineFft<N>::NI;
   const float2* T;
   float2 e, sg;    // exp(i C k) of the current item, exp(i C G)
   float dmr, tdr;  // multipliers per unit of n - (wrap): dm r_o 2 pi / N and 2 pi / N
@@ -176,7 +63,7 @@ struct LineChirp {
 template <int N, int MODE, class S>
 __device__ __forceinline__ void pass_line(const PassArgs& A, const PhaseCoef* coef, int u, int v,
                                           int j, const S& s0, const S& s1, float2* table) {
-  using L = PassLine<N>;
+  using L = LineFft<N>;
   constexpr int G = L::G, R1 = L::R1, NI = L::NI;
   constexpr bool kDual = (MODE == PM_DUAL_IN || MODE == PM_DUAL_OUT);
   const bool id0 = phase_is_identity(A.ph[0]), id1 = phase_is_identity(A.ph[1]);
@@ -186,8 +73,12 @@ __device__ __forceinline__ void pass_line(const PassArgs& A, const PhaseCoef* co
   // (the tables' readers of the previous line are past that line's last __syncwarp)
   if (sep0) ch0.init(A.ph[0], coef[0], r_o(A.ph[0]), j, A.scale, A.scale_lo, table);
   if (sep1) ch1.init(A.ph[1], coef[1], r_o(A.ph[1]), j, A.scale, A.scale_lo, table + G);
-  if (MODE != PM_INV) L::first(s0);
-  if (MODE == PM_DUAL_IN) L::first(s1);
+  auto load0 = [&](int r, int) { return s0.tab(r, 0); };
+  auto load1 = [&](int r, int) { return s1.tab(r, 0); };
+  auto store0 = [&](int r, int, float2 x) { s0.tab(r, 0) = x; };
+  auto store1 = [&](int r, int, float2 x) { s1.tab(r, 0) = x; };
+  if (MODE != PM_INV) L::template first<true>(s0, j, load0);
+  if (MODE == PM_DUAL_IN) L::template first<true>(s1, j, load1);
   // X (index k + R1 r) times the factors of phase 0 or 1, the form decided once per line
   auto factor = [&](const bool id, const bool sep, const LineChirp<N>& ch, const int q, int k,
                     float2 (&X)[G]) {
@@ -233,7 +124,7 @@ __device__ __forceinline__ void pass_line(const PassArgs& A, const PhaseCoef* co
       if (sep0) ch0.next();
     }
     __syncwarp();
-    if (MODE == PM_INV) L::last(s0);
+    if (MODE == PM_INV) L::template last<true>(s0, j, store0);
     return;
   }
 #pragma unroll
@@ -267,8 +158,8 @@ __device__ __forceinline__ void pass_line(const PassArgs& A, const PhaseCoef* co
     if (NI > 1 && sep1) ch1.next();
   }
   __syncwarp();
-  L::last(s0);
-  if (MODE == PM_DUAL_OUT) L::last(s1);
+  L::template last<true>(s0, j, store0);
+  if (MODE == PM_DUAL_OUT) L::template last<true>(s1, j, store1);
 }
 
 }  // namespace me

@@ -24,27 +24,30 @@ static double twiddle_gain(int n, int na, int nb) {
 }
 
 // The same for a register DFT (RDft, fft_reg.cuh): radices 2 and 4 are exact, a prime's
-// coefficients are its twiddles, a composite is two DFTs with twiddles between.
+// coefficients are its twiddles, a composite is two DFTs with twiddles between where its
+// factors are not coprime.
 static double radix_gain(int r) {
   if (r <= 2 || r == 4) return 1.0;
   static const int first[33] = {0, 0, 0, 0, 0, 0, 2, 0, 2, 3, 2, 0, 4, 0, 2, 3, 4,
-                                0, 2, 0, 4, 3, 2, 0, 4, 5, 2, 3, 4, 0, 5, 0, 4};
+                                0, 2, 0, 4, 3, 2, 0, 8, 5, 2, 3, 4, 0, 2, 0, 4};
   const int a = first[r];
   if (a == 0) return twiddle_gain(r, r, r);
-  return radix_gain(a) * radix_gain(r / a) * twiddle_gain(r, a, r / a);
+  const int b = r / a;
+  const bool coprime = (a % 2 || b % 2) && (a % 3 || b % 3) && (a % 5 || b % 5);
+  return radix_gain(a) * radix_gain(b) * (coprime ? 1.0 : twiddle_gain(r, a, b));
 }
 
-static double plan_gain(int n, bool sense) {
-  static std::atomic<double> known[2][ME_MAX_LINE + 1];
+double fft_pair_gain(int n) {
+  static std::atomic<double> known[ME_MAX_LINE + 1];
   if (n < 1 || n > ME_MAX_LINE) return 1.0;
-  double g = known[sense][n].load(std::memory_order_relaxed);
+  double g = known[n].load(std::memory_order_relaxed);
   if (g != 0.0) return g;
   int r1 = 0, r2 = 0;
   switch (n) {
-#define ME_GAIN_CASE(N, R1, R2)     \
-  case N:                           \
-    r2 = sense ? R2 : N <= 128 ? 8 : 16; \
-    r1 = N / r2;                    \
+#define ME_GAIN_CASE(N)       \
+  case N:                     \
+    r1 = LineFft<N>::R1;      \
+    r2 = LineFft<N>::G;       \
     break;
     ME_FAST_LENGTHS(ME_GAIN_CASE)
 #undef ME_GAIN_CASE
@@ -57,12 +60,9 @@ static double plan_gain(int n, bool sense) {
     }
   }
   g = r1 ? radix_gain(r1) * radix_gain(r2) * twiddle_gain(n, r1, r2) : 1.0;
-  known[sense][n].store(g, std::memory_order_relaxed);
+  known[n].store(g, std::memory_order_relaxed);
   return g;
 }
-
-double fft_pair_gain(int n) { return plan_gain(n, false); }
-double sense_fft_pair_gain(int n) { return plan_gain(n, true); }
 
 int try_rt_pass(int mode, PassArgs& A, cudaStream_t stream) {
   RtPlan P;

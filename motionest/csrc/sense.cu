@@ -17,7 +17,7 @@
 //                     K, IFFT_y, accumulates conj(mps) . h in registers, writes one image block.
 #include <algorithm>
 #include <cstdlib>
-#include <vector>
+#include <type_traits>
 
 #include "fft_reg.cuh"
 #include "line_pass.cuh"
@@ -32,10 +32,8 @@ namespace me {
     if (_rc != ME_OK) return _rc; \
   } while (0)
 
-// Resident CTAs per SM the fast SENSE kernels are compiled for (register budget 65536/(256*n)).
-#ifndef ME_SENSE_MINB
-#define ME_SENSE_MINB 2
-#endif
+// Resident CTAs per SM that the compile-time SENSE kernels are built for.
+__host__ __device__ constexpr int sense_min_ctas(int y) { return line_threads(y) == 8 ? 3 : 2; }
 
 // Gauss-Newton sums of one sample: |r|^2, Re(conj(r) J_p) and Re(conj(J_p) J_q) for q >= p.
 __device__ __forceinline__ void lm_accumulate(double (&st)[kLmStats], float2 r, const float2 (&J)[6]) {
@@ -232,7 +230,7 @@ __global__ void __launch_bounds__(kThreads) sense_adj_kernel(const AdjArgs A) {
 __device__ __forceinline__ void init_twiddles_any(float2* tw, int n) {
   const float2* g = nullptr;
   switch (n) {
-#define ME_TW_CASE(N, R1, R2) \
+#define ME_TW_CASE(N) \
   case N: g = tw##N; break;
     ME_FAST_LENGTHS(ME_TW_CASE)
 #undef ME_TW_CASE
@@ -245,22 +243,38 @@ __device__ __forceinline__ void init_twiddles_any(float2* tw, int n) {
   }
 }
 
+// Map and image rows go from L2 straight into the registers of the DFT that uses them (16 or 14
+// loads in flight per thread); staging them in shared memory first, by bulk copies, cost more in
+// shared-memory traffic than it hid: without it, and with the plans of LineFft, the forward went
+// from 55.8 to 53.5 ms and the adjoint from 63.6 to 60.8 ms at 256x224x176, 32 coils, 64 shots,
+// and from 2.50 to 1.68 and 3.47 to 2.10 ms at 128x112x88, 16 coils, 32 shots (three CTAs per SM
+// instead of two for the forward up to 128 points).  What bounds both: instruction issue and the
+// shared-memory pipe together (transposes, columns of the sample sums, H rows).
+
+// This thread's row group g and its place j < G in it: sixteen threads of one row to a half warp,
+// or eight of two.  (With half warps of two rows of 224 points the forward took 62.1 ms instead
+// of 56.8 ms.)
+template <int G>
+__device__ __forceinline__ void row_place(int& g, int& j) {
+  g = threadIdx.x / G;
+  j = threadIdx.x % G;
+}
+
 // Rows per chunk of the forward kernel (one row per thread group) and its shared-memory plan.
-template <int Y, int R1, int R2>
+template <int Y>
 struct FwdPlan {
-  using F = LineFft<Y, R1, R2>;
+  using F = LineFft<Y>;
   static constexpr int G = F::G;
   static constexpr int NG = kThreads / G;
   static constexpr int RC = NG;
-  static constexpr int LS = F::LS;
-  static constexpr int STAGE = 2 * RC * Y;  // staged map rows + image rows
+  static constexpr int LS = line_region(Y);
   static constexpr int LINES = NG * LS;
 };
 
-template <int Y, int R1, int R2, int MPT, int MODE>
-__global__ void __launch_bounds__(kThreads, ME_SENSE_MINB) fast_fwd_kernel(const FwdArgs A) {
+template <int Y, int MPT, int MODE>
+__global__ void __launch_bounds__(kThreads, sense_min_ctas(Y)) fast_fwd_kernel(const FwdArgs A) {
   static_assert(MODE == FWD_K || MODE == FWD_RESID, "one volume per CTA");
-  using P = FwdPlan<Y, R1, R2>;
+  using P = FwdPlan<Y>;
   using F = typename P::F;
   constexpr int G = P::G, RC = P::RC, LS = P::LS;
   static_assert(RC % 2 == 0, "the two Horner chains take rows in pairs");
@@ -271,8 +285,7 @@ __global__ void __launch_bounds__(kThreads, ME_SENSE_MINB) fast_fwd_kernel(const
   const int b = bx / A.vps, vk = bx - b * A.vps;  // shot in the batch, volume of the shot
   const int s = A.shot0 + b;
   const int X = A.X;
-  float2* stage = sm;                 // [2][RC][Y]: map rows, then image rows
-  float2* lines = stage + P::STAGE;   // one line region per thread group
+  float2* lines = sm;  // one line region per thread group
   float2* twX = lines + P::LINES;
   init_twiddles_any(twX, X);
 
@@ -295,44 +308,14 @@ __global__ void __launch_bounds__(kThreads, ME_SENSE_MINB) fast_fwd_kernel(const
     }
     acc[m] = make_float2(0.f, 0.f);
   }
-  const int g = threadIdx.x / G, j = threadIdx.x % G;
+  int g, j;
+  row_place<G>(g, j);
   const i64 plane = (i64)X * Y;
   const float2* mrow = A.mps + ((i64)z * A.C + c) * plane;
   const float2* vbase = A.vols + (i64)bx * A.vol_stride + (i64)z * plane;
+  PaddedSlots<Y> slots;
+  slots.init(lines + g * LS, j);
 
-  // stage rows [x0, x0 + RC) of the map and of the image: the rows of a chunk are contiguous
-  // both in the plane and in the stage, so each is one flat copy.  With A.bulk one thread
-  // issues the two as bulk copies on the TMA engine (completion counted on `full`); otherwise
-  // every thread issues 16-byte cp.async copies.
-  __shared__ __align__(8) uint64_t full;
-  const bool bulk = A.bulk != 0;
-  if (bulk && threadIdx.x == 0) {
-    mbar_init(&full, 1);
-    fence_mbar_init();
-  }
-  auto issue = [&](int x0) {
-    const float2* ms = mrow + (i64)x0 * Y;
-    const float2* us = vbase + (i64)x0 * Y;
-    if (bulk) {
-      if (threadIdx.x == 0) {
-        const unsigned bytes = (unsigned)(min(RC, X - x0) * Y * sizeof(float2));
-        fence_proxy_async_smem();
-        mbar_arrive_expect_tx(&full, 2 * bytes);
-        bulk_g2s(stage, ms, bytes, &full);
-        bulk_g2s(stage + RC * Y, us, bytes, &full);
-      }
-      return;
-    }
-    const int nq = min(RC, X - x0) * (Y / 2);  // 16-byte chunks
-    for (int q = threadIdx.x; q < nq; q += kThreads) {
-      cp_async16(stage + 2 * q, ms + 2 * q);
-      cp_async16(stage + RC * Y + 2 * q, us + 2 * q);
-    }
-    cp_async_commit();
-  };
-
-  issue(0);  // the barrier stays untouched by other threads until the __syncthreads below
-  unsigned fphase = 0;
   // The Horner steps W^kx and W^2kx do not change between chunks: with few samples per thread
   // they are read from the table once (registers), else once per chunk.
   constexpr bool kHoist = MPT <= 2;
@@ -349,27 +332,18 @@ __global__ void __launch_bounds__(kThreads, ME_SENSE_MINB) fast_fwd_kernel(const
   }
   for (int x0 = 0; x0 < X; x0 += RC) {
     const int nr = min(RC, X - x0);
-    if (bulk) {
-      mbar_wait_bounded(&full, fphase, WF_SENSE_FWD);
-      fphase ^= 1;
-    } else {
-      cp_async_wait_all();
-    }
-    __syncthreads();
+    if (x0 > 0) __syncthreads();
     {
-      // FFT of map row x image row, the product formed as the first stage loads it; rows past
+      // FFT of map row x image row, read and multiplied as the first stage needs them; rows past
       // nr transform zeros
-      float2* L = lines + g * LS;
-      const float2* ms = stage + g * Y;
-      const float2* us = stage + (RC + g) * Y;
+      const float2* ms = mrow + (i64)(x0 + g) * Y;
+      const float2* us = vbase + (i64)(x0 + g) * Y;
       const bool live = g < nr;
-      float2 Xr[R2];
-      F::forward_from([&](int n) { return live ? cmul(ms[n], us[n]) : make_float2(0.f, 0.f); },
-                      L, j, Xr);
-      F::store_spectrum(L, j, Xr);
+      F::forward(slots, j, [&](int, int n) {
+        return live ? cmul(ms[n], us[n]) : make_float2(0.f, 0.f);
+      });
     }
     __syncthreads();
-    if (x0 + RC < X) issue(x0 + RC);
     // Sample sums over the chunk's rows by Horner's rule, sum_row L[row] W^(kx row), then one
     // table twiddle W^(kx x0) per chunk.  Rows past nr hold zeros (zero lines transform to
     // zero), so every chunk runs all RC rows, in two interleaved chains (even and odd rows,
@@ -402,7 +376,7 @@ __global__ void __launch_bounds__(kThreads, ME_SENSE_MINB) fast_fwd_kernel(const
 #pragma unroll
     for (int m = 0; m < MPT; m++) {
       const int jj = threadIdx.x + m * kThreads;
-      if (jj < ns) A.kout[(i64)vk * A.kout_vs + base + jj] = cscale(acc[m], A.scale);
+      if (jj < ns) A.kout[(i64)vk * A.kout_vs + base + jj] = cscale2(acc[m], A.scale, A.scale_lo);
     }
   } else {
     const i64 base = (i64)soff * A.C * A.Z + zc * ns;
@@ -411,7 +385,7 @@ __global__ void __launch_bounds__(kThreads, ME_SENSE_MINB) fast_fwd_kernel(const
     for (int m = 0; m < MPT; m++) {
       const int jj = threadIdx.x + m * kThreads;
       if (jj < ns) {
-        const float2 r = csub(cscale(acc[m], A.scale), A.ydat[base + jj]);
+        const float2 r = csub(cscale2(acc[m], A.scale, A.scale_lo), A.ydat[base + jj]);
         e[0] += (double)r.x * r.x + (double)r.y * r.y;
       }
     }
@@ -426,9 +400,9 @@ __global__ void __launch_bounds__(kThreads, ME_SENSE_MINB) fast_fwd_kernel(const
 // J_p> and H_pq = Re<J_p, J_q> (transform_estimation.py:39-68) instead of being written out.
 // The sums per sample and their block reduction are those of lm_stats_kernel, in the same order,
 // so the statistics are bit-identical to the two-kernel path.
-template <int Y, int R1, int R2, int MPT>
-__global__ void __launch_bounds__(kThreads, ME_SENSE_MINB) fast_lm_kernel(const FwdArgs A) {
-  using P = FwdPlan<Y, R1, R2>;
+template <int Y, int MPT>
+__global__ void __launch_bounds__(kThreads, 2) fast_lm_kernel(const FwdArgs A) {
+  using P = FwdPlan<Y>;
   using F = typename P::F;
   constexpr int G = P::G, RC = P::RC, LS = P::LS;
   constexpr int NV = 7;
@@ -437,8 +411,7 @@ __global__ void __launch_bounds__(kThreads, ME_SENSE_MINB) fast_lm_kernel(const 
   const int b = blockIdx.x, c = blockIdx.y, z = blockIdx.z;
   const int s = A.shot0 + b;
   const int X = A.X;
-  float2* stage = sm;                // map rows [RC][Y], then one volume's image rows [RC][Y]
-  float2* lines = stage + P::STAGE;  // one line region per thread group
+  float2* lines = sm;  // one line region per thread group
   float2* twX = lines + P::LINES;
   init_twiddles_any(twX, X);
 
@@ -461,41 +434,14 @@ __global__ void __launch_bounds__(kThreads, ME_SENSE_MINB) fast_lm_kernel(const 
 #pragma unroll
     for (int v = 0; v < NV; v++) acc[v][m] = make_float2(0.f, 0.f);
   }
-  const int g = threadIdx.x / G, j = threadIdx.x % G;
+  int g, j;
+  row_place<G>(g, j);
   const i64 plane = (i64)X * Y;
   const float2* mrow = A.mps + ((i64)z * A.C + c) * plane;
   const float2* vbase = A.vols + (i64)b * NV * A.vol_stride + (i64)z * plane;
+  PaddedSlots<Y> slots;
+  slots.init(lines + g * LS, j);
 
-  // stage the image rows [x0, x0 + RC) of volume v, with the map rows too when `map`
-  __shared__ __align__(8) uint64_t full;
-  const bool bulk = A.bulk != 0;
-  if (bulk && threadIdx.x == 0) {
-    mbar_init(&full, 1);
-    fence_mbar_init();
-  }
-  auto issue = [&](int x0, int v, bool map) {
-    const float2* ms = mrow + (i64)x0 * Y;
-    const float2* us = vbase + (i64)v * A.vol_stride + (i64)x0 * Y;
-    if (bulk) {
-      if (threadIdx.x == 0) {
-        const unsigned bytes = (unsigned)(min(RC, X - x0) * Y * sizeof(float2));
-        fence_proxy_async_smem();
-        mbar_arrive_expect_tx(&full, map ? 2 * bytes : bytes);
-        if (map) bulk_g2s(stage, ms, bytes, &full);
-        bulk_g2s(stage + RC * Y, us, bytes, &full);
-      }
-      return;
-    }
-    const int nq = min(RC, X - x0) * (Y / 2);
-    for (int q = threadIdx.x; q < nq; q += kThreads) {
-      if (map) cp_async16(stage + 2 * q, ms + 2 * q);
-      cp_async16(stage + RC * Y + 2 * q, us + 2 * q);
-    }
-    cp_async_commit();
-  };
-
-  issue(0, 0, true);  // the barrier stays untouched by other threads until the __syncthreads below
-  unsigned fphase = 0;
   constexpr bool kHoist = MPT <= 2;
   float2 hst[kHoist ? MPT : 1], hst2[kHoist ? MPT : 1];
   __syncthreads();  // twX is written above by all threads
@@ -512,29 +458,16 @@ __global__ void __launch_bounds__(kThreads, ME_SENSE_MINB) fast_lm_kernel(const 
     const int nr = min(RC, X - x0);
 #pragma unroll 1
     for (int v = 0; v < NV; v++) {
-      if (bulk) {
-        mbar_wait_bounded(&full, fphase, WF_SENSE_FWD);
-        fphase ^= 1;
-      } else {
-        cp_async_wait_all();
-      }
       __syncthreads();
       {
-        float2* L = lines + g * LS;
-        const float2* ms = stage + g * Y;
-        const float2* us = stage + (RC + g) * Y;
+        const float2* ms = mrow + (i64)(x0 + g) * Y;
+        const float2* us = vbase + (i64)v * A.vol_stride + (i64)(x0 + g) * Y;
         const bool live = g < nr;
-        float2 Xr[R2];
-        F::forward_from([&](int n) { return live ? cmul(ms[n], us[n]) : make_float2(0.f, 0.f); },
-                        L, j, Xr);
-        F::store_spectrum(L, j, Xr);
+        F::forward(slots, j, [&](int, int n) {
+          return live ? cmul(ms[n], us[n]) : make_float2(0.f, 0.f);
+        });
       }
       __syncthreads();
-      if (v + 1 < NV) {
-        issue(x0, v + 1, false);
-      } else if (x0 + RC < X) {
-        issue(x0 + RC, 0, true);
-      }
       // sample sums of volume v over the chunk's rows (as fast_fwd_kernel)
 #pragma unroll
       for (int m = 0; m < MPT; m++) {
@@ -576,13 +509,12 @@ __global__ void __launch_bounds__(kThreads, ME_SENSE_MINB) fast_lm_kernel(const 
   for (int m = 0; m < MPT; m++) {
     const int jj = threadIdx.x + m * kThreads;
     if (jj < ns) {
-      // K rounded to float before the difference, as the two-kernel path stores it (a
-      // contracted multiply-subtract would round differently)
-      const float2 k0 = make_float2(__fmul_rn(acc[0][m].x, A.scale), __fmul_rn(acc[0][m].y, A.scale));
+      // K rounded to float before the difference, as the two-kernel path stores it
+      const float2 k0 = cscale2(acc[0][m], A.scale, A.scale_lo);
       const float2 r = csub(k0, A.ydat[yb + jj]);
       float2 J[6];
 #pragma unroll
-      for (int p = 0; p < 6; p++) J[p] = cscale(acc[1 + p][m], A.scale);
+      for (int p = 0; p < 6; p++) J[p] = cscale2(acc[1 + p][m], A.scale, A.scale_lo);
       lm_accumulate(st, r, J);
     }
   }
@@ -591,12 +523,12 @@ __global__ void __launch_bounds__(kThreads, ME_SENSE_MINB) fast_lm_kernel(const 
 
 // Adjoint plan: one image row per thread group; the H rows are built by one thread per ky bin
 // (and part of the rows), walking its samples with a twiddle recurrence along x.
-template <int Y, int R1, int R2>
+template <int Y>
 struct AdjPlan {
-  using F = LineFft<Y, R1, R2>;
+  using F = LineFft<Y>;
   static constexpr int G = F::G;
   static constexpr int NG = kThreads / G;
-  static constexpr int LS = F::LS;
+  static constexpr int LS = line_region(Y);
   static constexpr int NP0 = (kThreads / Y) < 1 ? 1 : (kThreads / Y);
   static constexpr int NPARTS = NP0 >= 16 ? 16 : NP0 >= 8 ? 8 : NP0 >= 4 ? 4 : NP0 >= 2 ? 2 : 1;
   static constexpr int RP = NG / NPARTS;  // rows per H-building thread
@@ -604,12 +536,16 @@ struct AdjPlan {
   // thread takes the second half of the rows of one of the heaviest bins (bins come sorted by
   // sample count), halving the longest walk; both halves write their own rows.
   static constexpr int NSPLIT = (NPARTS == 1 && Y < kThreads) ? (kThreads - Y < Y ? kThreads - Y : Y) : 0;
-  static constexpr int RH = RP / 2;  // rows of each half of a shared bin
+  static constexpr int RH = RP > 1 ? RP / 2 : 1;  // rows of each half of a shared bin
+  // first rows of the threads' row ranges: multiples of START_ROWS; tabulated as factors when few
+  static constexpr int START_ROWS = NSPLIT > 0 ? RH : RP;
+  static constexpr int STARTS = NSPLIT > 0 ? 2 : NPARTS;
+  static constexpr bool TABULATE = STARTS <= 2;
 };
 
-template <int Y, int R1, int R2>
-__global__ void __launch_bounds__(kThreads, ME_SENSE_MINB) fast_adj_kernel(const AdjArgs A) {
-  using P = AdjPlan<Y, R1, R2>;
+template <int Y>
+__global__ void __launch_bounds__(kThreads, Y <= 64 ? 3 : 2) fast_adj_kernel(const AdjArgs A) {
+  using P = AdjPlan<Y>;
   using F = typename P::F;
   constexpr int G = P::G, NG = P::NG, LS = P::LS, RP = P::RP, NSPLIT = P::NSPLIT;
   extern __shared__ __align__(16) float2 sm[];
@@ -619,33 +555,36 @@ __global__ void __launch_bounds__(kThreads, ME_SENSE_MINB) fast_adj_kernel(const
   const int X = A.X;
   const int soff = A.shot_off[s];
   const int ns = A.shot_off[s + 1] - soff;
-  const int kcap = (A.XB + 1) & ~1;            // max samples per shot, padded
-  float2* mstage = sm;                          // 2 x [NG][Y] maps rows
-  float2* Kb = mstage + 2 * NG * Y;             // 2 x kcap samples
-  float2* lines = Kb + 2 * kcap;                // NG x LS
+  const int kcap = (A.XB + 1) & ~1;   // max samples per shot, padded
+  float2* Kb = sm;                    // 2 x kcap samples
+  float2* lines = Kb + 2 * kcap;      // NG x LS
   float2* twX = lines + NG * LS;
-  // with NSPLIT > 0: per-sample twiddles shared by all coils, conj W^(kx x0), conj W^(kx (x0 +
-  // RH)) and conj W^kx
-  float2* tw_a = twX + pad2(X);
-  float2* tw_b = tw_a + kcap;
-  float2* tw_s = tw_b + kcap;
+  // per sample, shared by all coils: conj W^kx and, at the first row of each of the P::STARTS row
+  // ranges that threads build, conj W^(kx x) -- as factors, or (short lines, many ranges) as
+  // indices into twX
+  float2* tw_s = twX + pad2(X);
+  float2* tw_0 = tw_s + kcap;
+  unsigned short* ix_s = reinterpret_cast<unsigned short*>(tw_s);
+  unsigned short* ix_0 = ix_s + kcap;
   init_twiddles_any(twX, X);
 
-  const int g = threadIdx.x / G, j = threadIdx.x % G;
+  int g, j;
+  row_place<G>(g, j);
   const int x = x0 + g;
-  const int nrows = min(NG, X - x0);
+  const bool live = x < X;
   const float inv_x = 1.0f / (float)X;
   const int* kyo = A.ky_off + (i64)s * (Y + 1);
-  const int* kxs = A.kx + soff;
   const i64 kbase0 = (A.kin_rel ? (i64)(soff - A.shot_off[A.shot0]) : (i64)soff) * A.C * A.Z;
   const i64 plane = (i64)X * Y;
-  if constexpr (NSPLIT > 0) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < ns; i += kThreads) {
-      const int kx = kxs[i];
-      tw_s[i] = cconj(twX[kx]);
-      tw_a[i] = cconj(twX[mulmod(kx, min(x0, X - 1), X, inv_x)]);
-      tw_b[i] = cconj(twX[mulmod(kx, min(x0 + P::RH, X - 1), X, inv_x)]);
+  __syncthreads();
+  for (int i = threadIdx.x; i < ns; i += kThreads) {
+    const int kx = A.kx[soff + i];
+    if (P::TABULATE) tw_s[i] = cconj(twX[kx]);
+    else ix_s[i] = (unsigned short)kx;
+    for (int q = 0; q < P::STARTS; q++) {
+      const int xi = mulmod(kx, min(x0 + q * P::START_ROWS, X - 1), X, inv_x);
+      if (P::TABULATE) tw_0[q * kcap + i] = cconj(twX[xi]);
+      else ix_0[q * kcap + i] = (unsigned short)xi;
     }
   }
 
@@ -666,108 +605,61 @@ __global__ void __launch_bounds__(kThreads, ME_SENSE_MINB) fast_adj_kernel(const
     half = true;
   }
   const int hlo = hbuild ? kyo[hb] : 0, hhi = hbuild ? kyo[hb + 1] : 0;
+  const int start = (hr0 / P::START_ROWS) * kcap;
 
-  // map rows of coil c into buffer c & 1: with A.bulk one bulk copy on the TMA engine
-  // (completion counted on full[c & 1]), otherwise 16-byte cp.async copies; the coil's samples
-  // (8-byte aligned only) always by cp.async
-  __shared__ __align__(8) uint64_t full[2];
-  const bool bulk = A.bulk != 0;
-  if (bulk && threadIdx.x == 0) {
-    mbar_init(&full[0], 1);
-    mbar_init(&full[1], 1);
-    fence_mbar_init();
-  }
+  // coil c's samples into buffer c & 1
   auto issue = [&](int c) {
-    const float2* mr = A.mps + ((i64)z * A.C + c) * plane + (i64)x0 * Y;
-    float2* dst = mstage + (c & 1) * NG * Y;
-    if (bulk) {
-      if (threadIdx.x == 0) {
-        const unsigned bytes = (unsigned)(nrows * Y * sizeof(float2));
-        fence_proxy_async_smem();
-        mbar_arrive_expect_tx(&full[c & 1], bytes);
-        bulk_g2s(dst, mr, bytes, &full[c & 1]);
-      }
-    } else {
-      const int nq = nrows * Y / 2;
-      for (int q = threadIdx.x; q < nq; q += kThreads) cp_async16(dst + 2 * q, mr + 2 * q);
-    }
     const float2* kc = A.kin + kbase0 + ((i64)z * A.C + c) * ns;
     float2* kd = Kb + (c & 1) * kcap;
     for (int i = threadIdx.x; i < ns; i += kThreads) cp_async8(kd + i, kc + i);
     cp_async_commit();
   };
 
-  // image row accumulators in the inverse FFT's output layout: thread j < R2 owns y = j + b R2
-  float2 w[R1];
+  // image row accumulators in the inverse FFT's output layout: thread j owns y = j + G q
+  float2 w[F::R1];
 #pragma unroll
-  for (int m = 0; m < R1; m++) w[m] = make_float2(0.f, 0.f);
-  float2* L = lines + g * LS;
+  for (int m = 0; m < F::R1; m++) w[m] = make_float2(0.f, 0.f);
+  PaddedSlots<Y> slots;
+  slots.init(lines + g * LS, j);
 
-  if (bulk) __syncthreads();  // the barriers are initialised before any thread waits on them
   issue(0);
   for (int c = 0; c < A.C; c++) {
     cp_async_wait_all();
-    if (bulk) mbar_wait_bounded(&full[c & 1], (c >> 1) & 1, WF_SENSE_ADJ);
     __syncthreads();
     if (c + 1 < A.C) issue(c + 1);
     const float2* K = Kb + (c & 1) * kcap;
+    const float2* ms = A.mps + ((i64)z * A.C + c) * plane + (i64)x * Y + j;
     if (hbuild) {
       // H[x][ky] += K exp(+2 pi i kx x / X): the term itself steps by conj(W^kx) per row
       float2 h[RP];
 #pragma unroll
       for (int r = 0; r < RP; r++) h[r] = make_float2(0.f, 0.f);
-      if constexpr (NSPLIT > 0) {
-        const float2* tw0 = (hr0 == 0) ? tw_a : tw_b;
-        if (half) {
-          for (int i = hlo; i < hhi; i++) {
-            const float2 st = tw_s[i];
-            float2 v = cmul(K[i], tw0[i]);
-#pragma unroll
-            for (int r = 0; r < P::RH; r++) {
-              h[r] = cadd(h[r], v);
-              v = cmul(v, st);
-            }
-          }
-#pragma unroll
-          for (int r = 0; r < P::RH; r++) lines[(hr0 + r) * LS + hb] = h[r];
-        } else {
-          for (int i = hlo; i < hhi; i++) {
-            const float2 st = tw_s[i];
-            float2 v = cmul(K[i], tw0[i]);
-#pragma unroll
-            for (int r = 0; r < RP; r++) {
-              h[r] = cadd(h[r], v);
-              v = cmul(v, st);
-            }
-          }
-#pragma unroll
-          for (int r = 0; r < RP; r++) lines[(hr0 + r) * LS + hb] = h[r];
-        }
-      } else {
+      auto walk = [&](auto rows) {
+        constexpr int ROWS = decltype(rows)::value;
         for (int i = hlo; i < hhi; i++) {
-          const int kx = kxs[i];
-          const float2 st = twX[kx];
-          float2 v = cmulc(K[i], twX[mulmod(kx, min(x0 + hr0, X - 1), X, inv_x)]);
+          const float2 st = P::TABULATE ? tw_s[i] : cconj(twX[ix_s[i]]);
+          float2 v = cmul(K[i], P::TABULATE ? tw_0[start + i] : cconj(twX[ix_0[start + i]]));
 #pragma unroll
-          for (int r = 0; r < RP; r++) {
+          for (int r = 0; r < ROWS; r++) {
             h[r] = cadd(h[r], v);
-            v = cmulc(v, st);
+            v = cmul(v, st);
           }
         }
 #pragma unroll
-        for (int r = 0; r < RP; r++) lines[(hr0 + r) * LS + hb] = h[r];
-      }
+        for (int r = 0; r < ROWS; r++) lines[(hr0 + r) * LS + hb] = h[r];
+      };
+      if (NSPLIT > 0 && half) walk(std::integral_constant<int, P::RH>{});
+      else walk(std::integral_constant<int, RP>{});
     }
     __syncthreads();
-    float2 Xr[R2];
-    F::load_spectrum(L, j, Xr);
-    const float2* ms = mstage + (c & 1) * NG * Y + g * Y;
-    F::inverse_to(L, j, Xr, [&](int q, int y, float2 v) { w[q] = cadd(w[q], cmulc(v, ms[y])); });
+    F::inverse(slots, j, [&](int q, int, float2 v) {
+      if (live) w[q] = cadd(w[q], cmulc(v, __ldg(ms + q * G)));
+    });
   }
-  if (g < nrows && j < R2) {
-    float2* o = A.out + (i64)b * A.vol_stride + (i64)z * plane + (i64)x * Y;
+  if (live) {
+    float2* o = A.out + (i64)b * A.vol_stride + (i64)z * plane + (i64)x * Y + j;
 #pragma unroll
-    for (int q = 0; q < R1; q++) o[j + q * R2] = cscale(w[q], A.scale);
+    for (int q = 0; q < F::R1; q++) o[q * G] = cscale2(w[q], A.scale, A.scale_lo);
   }
 }
 
@@ -1047,7 +939,7 @@ static bool fast_sense_enabled() {
 
 // 1/sqrt(XY), with the gain of the FFT along y taken out
 static double sense_scale(const me_sense* pb) {
-  return 1.0 / sqrt((double)pb->nx * pb->ny * (fast_sense_enabled() ? sense_fft_pair_gain(pb->ny) : 1.0));
+  return 1.0 / sqrt((double)pb->nx * pb->ny * (fast_sense_enabled() ? fft_pair_gain(pb->ny) : 1.0));
 }
 
 static int fwd_rows(int V, int Y) {
@@ -1075,18 +967,6 @@ static int launch_fwd_v(FwdArgs& A, int maxps, int nb, cudaStream_t st) {
   return launch_fwd_t<8, V, MODE>(A, nb, st);
 }
 
-// Row staging by bulk copies (TMA engine) unless ME_NO_BULK=1; used where every staged range
-// starts on a 16-byte boundary.
-static bool bulk_enabled() {
-  static int v = -1;
-  if (v < 0) {
-    const char* e = getenv("ME_NO_BULK");
-    v = (e && e[0] == '1') ? 0 : 1;
-  }
-  return v == 1;
-}
-static bool al16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
-
 ME_WAIT_FAULT_ACCESSOR(sense_wait_fault)
 
 // The LM statistics from the fused seven-volume kernel unless ME_LM_TWO_PASS=1 (the forward
@@ -1100,49 +980,49 @@ static bool fused_lm_enabled() {
   return v == 1;
 }
 
-template <int Y, int R1, int R2, int MPT, int MODE>
+template <int Y, int MPT, int MODE>
 static int launch_fast_fwd_t(FwdArgs& A, int nb, cudaStream_t st) {
-  using P = FwdPlan<Y, R1, R2>;
-  const size_t smem = sizeof(float2) * ((size_t)P::STAGE + P::LINES + pad2(A.X));
-  ME_TRY(check_cuda(allow_smem(fast_fwd_kernel<Y, R1, R2, MPT, MODE>, smem), "fwd smem"));
+  using P = FwdPlan<Y>;
+  const size_t smem = sizeof(float2) * ((size_t)P::LINES + pad2(A.X));
+  ME_TRY(check_cuda(allow_smem(fast_fwd_kernel<Y, MPT, MODE>, smem), "fwd smem"));
   dim3 grid(nb * A.vps, A.C, A.Z);
   count_launch();
-  fast_fwd_kernel<Y, R1, R2, MPT, MODE><<<grid, kThreads, smem, st>>>(A);
+  fast_fwd_kernel<Y, MPT, MODE><<<grid, kThreads, smem, st>>>(A);
   return check_cuda(cudaGetLastError(), "fast sense_fwd launch");
 }
 
-template <int Y, int R1, int R2, int MODE>
+template <int Y, int MODE>
 static int launch_fast_fwd_m(FwdArgs& A, int maxps, int nb, cudaStream_t st) {
-  if (maxps <= kThreads) return launch_fast_fwd_t<Y, R1, R2, 1, MODE>(A, nb, st);
-  if (maxps <= 2 * kThreads) return launch_fast_fwd_t<Y, R1, R2, 2, MODE>(A, nb, st);
-  if (maxps <= 4 * kThreads) return launch_fast_fwd_t<Y, R1, R2, 4, MODE>(A, nb, st);
-  return launch_fast_fwd_t<Y, R1, R2, 8, MODE>(A, nb, st);
+  if (maxps <= kThreads) return launch_fast_fwd_t<Y, 1, MODE>(A, nb, st);
+  if (maxps <= 2 * kThreads) return launch_fast_fwd_t<Y, 2, MODE>(A, nb, st);
+  if (maxps <= 4 * kThreads) return launch_fast_fwd_t<Y, 4, MODE>(A, nb, st);
+  return launch_fast_fwd_t<Y, 8, MODE>(A, nb, st);
 }
 
-template <int Y, int R1, int R2, int MPT>
+template <int Y, int MPT>
 static int launch_fast_lm_t(FwdArgs& A, int nb, cudaStream_t st) {
-  using P = FwdPlan<Y, R1, R2>;
-  const size_t smem = sizeof(float2) * ((size_t)P::STAGE + P::LINES + pad2(A.X));
-  ME_TRY(check_cuda(allow_smem(fast_lm_kernel<Y, R1, R2, MPT>, smem), "lm smem"));
+  using P = FwdPlan<Y>;
+  const size_t smem = sizeof(float2) * ((size_t)P::LINES + pad2(A.X));
+  ME_TRY(check_cuda(allow_smem(fast_lm_kernel<Y, MPT>, smem), "lm smem"));
   dim3 grid(nb, A.C, A.Z);
   count_launch();
-  fast_lm_kernel<Y, R1, R2, MPT><<<grid, kThreads, smem, st>>>(A);
+  fast_lm_kernel<Y, MPT><<<grid, kThreads, smem, st>>>(A);
   return check_cuda(cudaGetLastError(), "fast lm launch");
 }
 
 // The fused statistics kernel keeps seven accumulators per sample in registers: up to two
 // samples per thread (512 per shot); more take the two-kernel path.
-template <int Y, int R1, int R2>
+template <int Y>
 static int launch_fast_lm_y(FwdArgs& A, int maxps, int nb, cudaStream_t st) {
-  if (maxps <= kThreads) return launch_fast_lm_t<Y, R1, R2, 1>(A, nb, st);
-  if (maxps <= 2 * kThreads) return launch_fast_lm_t<Y, R1, R2, 2>(A, nb, st);
+  if (maxps <= kThreads) return launch_fast_lm_t<Y, 1>(A, nb, st);
+  if (maxps <= 2 * kThreads) return launch_fast_lm_t<Y, 2>(A, nb, st);
   return -1;
 }
 
 static int try_fast_lm(FwdArgs& A, int maxps, int nb, cudaStream_t st) {
   switch (A.Y) {
-#define ME_LM_CASE(N, R1, R2) \
-  case N: return launch_fast_lm_y<N, R1, R2>(A, maxps, nb, st);
+#define ME_LM_CASE(N) \
+  case N: return launch_fast_lm_y<N>(A, maxps, nb, st);
     ME_FAST_LENGTHS(ME_LM_CASE)
 #undef ME_LM_CASE
     default: return -1;
@@ -1151,42 +1031,42 @@ static int try_fast_lm(FwdArgs& A, int maxps, int nb, cudaStream_t st) {
 
 // The compile-time kernels take one volume per CTA (FWD_K, FWD_RESID); the seven-volume LM
 // statistics use FWD_K over seven volumes per shot and lm_stats_kernel instead of FWD_LM.
-template <int Y, int R1, int R2>
+template <int Y>
 static int launch_fast_fwd_y(FwdArgs& A, int mode, int maxps, int nb, cudaStream_t st) {
-  if (mode == FWD_K) return launch_fast_fwd_m<Y, R1, R2, FWD_K>(A, maxps, nb, st);
-  if (mode == FWD_RESID) return launch_fast_fwd_m<Y, R1, R2, FWD_RESID>(A, maxps, nb, st);
+  if (mode == FWD_K) return launch_fast_fwd_m<Y, FWD_K>(A, maxps, nb, st);
+  if (mode == FWD_RESID) return launch_fast_fwd_m<Y, FWD_RESID>(A, maxps, nb, st);
   return -1;
 }
 
 static int try_fast_fwd(FwdArgs& A, int mode, int maxps, int nb, cudaStream_t st) {
   switch (A.Y) {
-#define ME_FWD_CASE(N, R1, R2) \
-  case N: return launch_fast_fwd_y<N, R1, R2>(A, mode, maxps, nb, st);
+#define ME_FWD_CASE(N) \
+  case N: return launch_fast_fwd_y<N>(A, mode, maxps, nb, st);
     ME_FAST_LENGTHS(ME_FWD_CASE)
 #undef ME_FWD_CASE
     default: return -1;
   }
 }
 
-template <int Y, int R1, int R2>
+template <int Y>
 static int launch_fast_adj_y(AdjArgs& A, int maxps, int nb, cudaStream_t st) {
-  using P = AdjPlan<Y, R1, R2>;
+  using P = AdjPlan<Y>;
   constexpr int NG = P::NG;
   A.XB = maxps;
-  const size_t smem = sizeof(float2) * (2 * (size_t)NG * Y + 2 * (size_t)pad2(maxps) +
-                                        (size_t)NG * P::LS + pad2(A.X) +
-                                        (P::NSPLIT > 0 ? 3 * (size_t)pad2(maxps) : 0));
-  ME_TRY(check_cuda(allow_smem(fast_adj_kernel<Y, R1, R2>, smem), "adj smem"));
+  const size_t kcap = pad2(maxps);
+  const size_t smem = sizeof(float2) * (2 * kcap + (size_t)NG * P::LS + pad2(A.X)) +
+                      (1 + P::STARTS) * kcap * (P::TABULATE ? sizeof(float2) : sizeof(short));
+  ME_TRY(check_cuda(allow_smem(fast_adj_kernel<Y>, smem), "adj smem"));
   dim3 grid(nb, (A.X + NG - 1) / NG, A.Z);
   count_launch();
-  fast_adj_kernel<Y, R1, R2><<<grid, kThreads, smem, st>>>(A);
+  fast_adj_kernel<Y><<<grid, kThreads, smem, st>>>(A);
   return check_cuda(cudaGetLastError(), "fast sense_adj launch");
 }
 
 static int try_fast_adj(AdjArgs& A, int maxps, int nb, cudaStream_t st) {
   switch (A.Y) {
-#define ME_ADJ_CASE(N, R1, R2) \
-  case N: return launch_fast_adj_y<N, R1, R2>(A, maxps, nb, st);
+#define ME_ADJ_CASE(N) \
+  case N: return launch_fast_adj_y<N>(A, maxps, nb, st);
     ME_FAST_LENGTHS(ME_ADJ_CASE)
 #undef ME_ADJ_CASE
     default: return -1;
@@ -1195,7 +1075,7 @@ static int try_fast_adj(AdjArgs& A, int maxps, int nb, cudaStream_t st) {
 
 static bool has_fast_length(int n) {
   switch (n) {
-#define ME_HAS_CASE(N, R1, R2) \
+#define ME_HAS_CASE(N) \
   case N: return true;
     ME_FAST_LENGTHS(ME_HAS_CASE)
 #undef ME_HAS_CASE
@@ -1239,8 +1119,6 @@ static int launch_fwd(const me_sense* pb, int mode, const float2* vols, i64 vol_
     return ME_ERR_UNSUPPORTED;
   }
   const int maxps = pb->samples.max_per_shot;
-  A.bulk = bulk_enabled() && al16(A.mps) && al16(A.vols) && vol_stride % 2 == 0 &&
-           pb->ny % 2 == 0;
   if (fast_sense_enabled() && pb->nx <= 512) {
     // FWD_LM over the seven volumes of each shot: the fused statistics kernel, or -1 (not
     // handled) for the caller's two-kernel path
@@ -1303,7 +1181,6 @@ static int launch_adj(const me_sense* pb, const float2* kin, int kin_rel, float2
     set_error("ny has a prime factor > 13");
     return ME_ERR_UNSUPPORTED;
   }
-  A.bulk = bulk_enabled() && al16(A.mps) && pb->ny % 2 == 0;
   if (fast_sense_enabled() && pb->nx <= 512) {
     int rc = try_fast_adj(A, pb->samples.max_per_shot, nb, st);
     if (rc < 0) rc = try_rt_adj(A, pb->samples.max_per_shot, nb, st);

@@ -28,7 +28,6 @@ struct FwdArgs {
   double* partial;
   int XR, es;
   float scale, scale_lo;  // 1/sqrt(XY) and what its rounding to float left
-  int bulk;  // stage rows with bulk copies (bases 16-byte aligned; set on the host)
   FftPlan plan;
 };
 
@@ -65,7 +64,6 @@ struct AdjArgs {
   const int* ky_order;  // may be null
   int XB, es;
   float scale, scale_lo;
-  int bulk;  // stage map rows with bulk copies (bases 16-byte aligned; set on the host)
   FftPlan plan;
 };
 
