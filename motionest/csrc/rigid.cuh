@@ -32,9 +32,13 @@ struct Rigid {
   // must run along it (kTanAxis[r]).
   int rotation(int r, const float2* in, i64 in_vs, float2* out, i64 out_vs, int nvol,
                int trans_axis = -1);
+  // rotated (may be null): R_r in, which the derivative's shears give on the way
   int rotation_derivative(int r, const float2* in, i64 in_vs, float2* out, i64 out_vs,
-                          float2* wa, float2* wb, i64 w_vs, int nvol, int trans_axis = -1);
-  int translation(const float2* in, i64 in_vs, float2* out, i64 out_vs, int deriv_axis, int nvol);
+                          float2* wa, float2* wb, i64 w_vs, int nvol, int trans_axis = -1,
+                          float2* rotated = nullptr, i64 rotated_vs = 0);
+  // the three ramps, the one along skip_axis left out, the one along deriv_axis differentiated
+  int translation(const float2* in, i64 in_vs, float2* out, i64 out_vs, int deriv_axis, int nvol,
+                  int skip_axis = -1);
   int derivative(const float2* in, float2* out, int p, int mode, float2* wa, float2* wb);
   // For each of nvol volumes v: out_v[0] = T in_v, out_v[1+p] = dT/dp in_v, where out_v[k] =
   // out + v * out_bs + k * out_ks; work holds 5 volumes per v at work + v * work_bs.
