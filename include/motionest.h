@@ -206,6 +206,14 @@ typedef struct me_sense {
   const double* transforms;
 } me_sense;
 
+/* Host side of me_samples: the sample lists of nshots plane masks [nx][ny] (bytes, non-zero =
+ * sampled; HOST pointers all).  Each shot's samples sorted by ky, then kx: shot_off[nshots + 1],
+ * kx and ky [total], ky_off [nshots][ny + 1]; ky_order [nshots][ny] lists the shot's bins by
+ * decreasing sample count, bins of one count spread over residues mod 16.  `total` is the number
+ * of non-zero mask entries. */
+int me_sample_lists(const unsigned char* planes, int nshots, int nx, int ny, long long total,
+                    int* shot_off, int* kx, int* ky, int* ky_off, int* ky_order);
+
 /* Scratch needed by me_sense_normal / me_sense_rhs / me_sense_residual /
  * me_sense_residual_norms for a given batch
  * (bytes), and by me_lm_normal_equations (which holds, per shot of the batch, T x and its six

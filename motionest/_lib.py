@@ -85,6 +85,8 @@ _SIGS = {
                                            ctypes.c_int, ctypes.c_int, c_ptr, c_ptr]),
     "me_rigid_jacobian": (ctypes.c_int, [c_ptr, c_ptr, c_i64, MeLayout, ctypes.POINTER(MeGrid),
                                          c_ptr, ctypes.c_int, c_ptr, c_ptr]),
+    "me_sample_lists": (ctypes.c_int, [c_ptr, ctypes.c_int, ctypes.c_int, ctypes.c_int, c_i64,
+                                       c_ptr, c_ptr, c_ptr, c_ptr, c_ptr]),
     "me_sense_workspace_bytes": (c_i64, [ctypes.POINTER(MeSense), ctypes.c_int]),
     "me_lm_workspace_bytes": (c_i64, [ctypes.POINTER(MeSense), ctypes.c_int]),
     "me_sense_precond": (ctypes.c_int, [c_ptr, ctypes.c_int, ctypes.c_int, ctypes.c_int,

@@ -12,6 +12,8 @@ from math import ceil
 
 import numpy as np
 
+from . import _lib
+
 
 @dataclass
 class DisorderConfig:
@@ -106,36 +108,61 @@ class SampleLists:
     me_samples struct of the C ABI describes them."""
 
     def __init__(self, planes):
-        planes = np.asarray(planes, dtype=bool)
+        planes = np.ascontiguousarray(planes, dtype=bool)
         S, X, Y = planes.shape
-        kx_all, ky_all, off, kyoff = [], [], [0], []
-        for s in range(S):
-            kx, ky = np.nonzero(planes[s])
-            order = np.lexsort((kx, ky))
-            kx, ky = kx[order], ky[order]
-            kx_all.append(kx)
-            ky_all.append(ky)
-            off.append(off[-1] + kx.size)
-            kyoff.append(np.searchsorted(ky, np.arange(Y + 1), side="left"))
         self.nshots, self.nx, self.ny = S, X, Y
-        self.shot_off = np.asarray(off, dtype=np.int32)
-        self.kx = np.concatenate(kx_all).astype(np.int32) if S else np.zeros(0, np.int32)
-        self.ky = np.concatenate(ky_all).astype(np.int32) if S else np.zeros(0, np.int32)
-        self.ky_off = np.stack(kyoff).astype(np.int32).reshape(-1)
+        lists = _native_lists(planes)
+        if lists is None:
+            lists = _python_lists(planes)
+        self.shot_off, self.kx, self.ky, self.ky_off, self.ky_order = lists
         counts = np.diff(self.shot_off)
         self.max_per_shot = int(counts.max()) if S else 0
         self.total = int(self.shot_off[-1])
-        # bins of each shot by decreasing sample count (stable), for load-balanced adjoints,
-        # spread over bank residues within each run of equal counts
-        bins = np.diff(self.ky_off.reshape(S, Y + 1), axis=1)
-        # With 128 < Y < 256 the adjoint's 256 threads hold one bin each and the 256 - Y spare
-        # threads take the second halves of the first 256 - Y bins of this order, which are
-        # then built as two halves of 8 rows.
-        split = 256 - Y if 128 < Y < 256 else 0
-        order = np.argsort(-bins, axis=1, kind="stable")
-        self.ky_order = np.stack([spread_residues(o, b[o], split=split)
-                                  for o, b in zip(order, bins)]
-                                 ).astype(np.int32).reshape(-1) if S else order.reshape(-1)
+
+
+def _native_lists(planes):
+    """The lists by the library's me_sample_lists; None where the library is not built."""
+    try:
+        lib = _lib.load()
+    except (_lib.MotionEstError, OSError):
+        return None
+    S, X, Y = planes.shape
+    total = int(np.count_nonzero(planes))
+    out = [np.empty(n, np.int32) for n in (S + 1, total, total, S * (Y + 1), S * Y)]
+    if S == 0 or X == 0 or Y == 0 or total > np.iinfo(np.int32).max:
+        return None
+    _lib.check(lib.me_sample_lists(planes.ctypes.data, S, X, Y, total,
+                                   *(a.ctypes.data for a in out)))
+    return out
+
+
+def _python_lists(planes):
+    """The lists in Python: the meaning of me_sample_lists, and its stand-in."""
+    S, X, Y = planes.shape
+    kx_all, ky_all, off, kyoff = [], [], [0], []
+    for s in range(S):
+        kx, ky = np.nonzero(planes[s])
+        order = np.lexsort((kx, ky))
+        kx, ky = kx[order], ky[order]
+        kx_all.append(kx)
+        ky_all.append(ky)
+        off.append(off[-1] + kx.size)
+        kyoff.append(np.searchsorted(ky, np.arange(Y + 1), side="left"))
+    shot_off = np.asarray(off, dtype=np.int32)
+    kx = np.concatenate(kx_all).astype(np.int32) if S else np.zeros(0, np.int32)
+    ky = np.concatenate(ky_all).astype(np.int32) if S else np.zeros(0, np.int32)
+    ky_off = np.stack(kyoff).astype(np.int32).reshape(-1)
+    # bins of each shot by decreasing sample count (stable), for load-balanced adjoints,
+    # spread over bank residues within each run of equal counts
+    bins = np.diff(ky_off.reshape(S, Y + 1), axis=1)
+    # With 128 < Y < 256 the adjoint's 256 threads hold one bin each and the 256 - Y spare
+    # threads take the second halves of the first 256 - Y bins of this order, which are
+    # then built as two halves of 8 rows.
+    split = 256 - Y if 128 < Y < 256 else 0
+    order = np.argsort(-bins, axis=1, kind="stable")
+    ky_order = np.stack([spread_residues(o, b[o], split=split) for o, b in zip(order, bins)]
+                        ).astype(np.int32).reshape(-1) if S else order.reshape(-1)
+    return shot_off, kx, ky, ky_off, ky_order
 
 
 def spread_residues(order, counts, width=16, split=0):

@@ -122,3 +122,21 @@ def test_adjoint_bin_order_keeps_counts_and_spreads_residues():
                 new += np.bincount(order[s][w:w + 16] % 16, minlength=16).max()
                 old += np.bincount(plain[s][w:w + 16] % 16, minlength=16).max()
         assert new <= old, (X, Y, new, old)
+
+
+@pytest.mark.parametrize("S,X,Y,share", [(1, 1, 1, 1.0), (3, 5, 7, 0.4), (4, 16, 12, 0.0),
+                                         (2, 40, 128, 0.1), (3, 33, 129, 0.05), (5, 64, 224, 0.01),
+                                         (2, 20, 255, 0.3), (2, 9, 256, 0.5), (2, 8, 300, 0.2)])
+def test_native_lists_match_python(S, X, Y, share):
+    """me_sample_lists against the Python lists, element by element: empty shots, single points,
+    widths on both sides of the split rule (128 < Y < 256)."""
+    from motionest.sampling import _native_lists, _python_lists
+    rng = np.random.default_rng(S * X + Y)
+    planes = rng.random((S, X, Y)) < share
+    if S > 2:
+        planes[1] = False
+    got, want = _native_lists(planes), _python_lists(planes)
+    assert got is not None
+    for a, b in zip(got, want):
+        assert a.dtype == np.int32
+        np.testing.assert_array_equal(a, b)
