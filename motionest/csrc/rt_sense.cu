@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   float2* H = Kb + 2 * kcap;  // [NR][ys]
   float2* tab = H + NR * T.ys;
   unsigned short* skx = (unsigned short*)(tab + NR * T.ls);  // kx of a sample, and the index
-  unsigned short* sst = skx + kcap;                          // kx x mod X at each octet's start
+  unsigned short* sst = skx + kcap;                          // kx x mod X at each octet's middle
   rt_init_twiddles(tw, P);
   init_twiddles(twX, X);
   const float inv_x = 1.0f / (float)X;
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     const int kx = A.kx[soff + i];
     skx[i] = (unsigned short)kx;
     for (int o = 0; o < no; o++)
-      sst[o * kcap + i] = (unsigned short)mulmod(kx, min(x0 + o * kOctet, X - 1), X, inv_x);
+      sst[o * kcap + i] = (unsigned short)mulmod(kx, (x0 + o * kOctet + kOctet / 2) % X, X, inv_x);
   }
   const int* kyo = A.ky_off + (i64)s * (Y + 1);
   const int* order = A.ky_order ? A.ky_order + (i64)s * Y : nullptr;
@@ -214,26 +214,17 @@ __global__ void __launch_bounds__(kThreads, 2)
     __syncthreads();
     if (c + 1 < A.C) issue(c + 1);
     const float2* K = Kb + (c & 1) * kcap;
-    // H[x][ky] += K exp(+2 pi i kx x / X), eight rows of one bin per item, heaviest bins first:
-    // the term itself steps by conj(W^kx) per row
+    // H[x][ky] += K exp(+2 pi i kx x / X), eight rows of one bin per item, heaviest bins first
     for (int q = tid; q < Y * no; q += kThreads) {
       const int slot = q / no, o = q - slot * no;
       const int bin = order ? order[slot] : slot;
-      float2 h[kOctet];
-#pragma unroll
-      for (int r = 0; r < kOctet; r++) h[r] = make_float2(0.f, 0.f);
-      const int hi = kyo[bin + 1];
-      for (int i = kyo[bin]; i < hi; i++) {
-        const float2 st = twX[skx[i]];
-        float2 v = cmulc(K[i], twX[sst[o * kcap + i]]);
-#pragma unroll
-        for (int r = 0; r < kOctet; r++) {
-          h[r] = cadd(h[r], v);
-          v = cmulc(v, st);
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < kOctet; r++) H[(o * kOctet + r) * T.ys + bin] = h[r];
+      h_rows<kOctet>(
+          kyo[bin], kyo[bin + 1],
+          [&](int i, float2& v, float2& st) {
+            st = cconj(twX[skx[i]]);
+            v = cmulc(K[i], twX[sst[o * kcap + i]]);
+          },
+          [&](int r, float2 h) { H[(o * kOctet + r) * T.ys + bin] = h; });
     }
     __syncthreads();
     if (has2) {

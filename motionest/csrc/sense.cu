@@ -537,10 +537,13 @@ struct AdjPlan {
   // sample count), halving the longest walk; both halves write their own rows.
   static constexpr int NSPLIT = (NPARTS == 1 && Y < kThreads) ? (kThreads - Y < Y ? kThreads - Y : Y) : 0;
   static constexpr int RH = RP > 1 ? RP / 2 : 1;  // rows of each half of a shared bin
-  // first rows of the threads' row ranges: multiples of START_ROWS; tabulated as factors when few
-  static constexpr int START_ROWS = NSPLIT > 0 ? RH : RP;
-  static constexpr int STARTS = NSPLIT > 0 ? 2 : NPARTS;
-  static constexpr bool TABULATE = STARTS <= 2;
+  // middle rows of the threads' row ranges (whole ranges, or the whole and the two halves of a
+  // shared bin); their sample twiddles are tabulated as factors when they are few
+  static constexpr int STARTS = NSPLIT > 0 ? 3 : NPARTS;
+  static constexpr bool TABULATE = STARTS <= 3;
+  static __host__ __device__ constexpr int start_row(int q) {
+    return NSPLIT > 0 ? (q == 0 ? RH : q == 1 ? RH / 2 : RH + RH / 2) : q * RP + RP / 2;
+  }
 };
 
 template <int Y>
@@ -559,7 +562,7 @@ __global__ void __launch_bounds__(kThreads, Y <= 64 ? 3 : 2) fast_adj_kernel(con
   float2* Kb = sm;                    // 2 x kcap samples
   float2* lines = Kb + 2 * kcap;      // NG x LS
   float2* twX = lines + NG * LS;
-  // per sample, shared by all coils: conj W^kx and, at the first row of each of the P::STARTS row
+  // per sample, shared by all coils: conj W^kx and, at the middle row of each of the P::STARTS row
   // ranges that threads build, conj W^(kx x) -- as factors, or (short lines, many ranges) as
   // indices into twX
   float2* tw_s = twX + pad2(X);
@@ -582,7 +585,7 @@ __global__ void __launch_bounds__(kThreads, Y <= 64 ? 3 : 2) fast_adj_kernel(con
     if (P::TABULATE) tw_s[i] = cconj(twX[kx]);
     else ix_s[i] = (unsigned short)kx;
     for (int q = 0; q < P::STARTS; q++) {
-      const int xi = mulmod(kx, min(x0 + q * P::START_ROWS, X - 1), X, inv_x);
+      const int xi = mulmod(kx, (x0 + P::start_row(q)) % X, X, inv_x);
       if (P::TABULATE) tw_0[q * kcap + i] = cconj(twX[xi]);
       else ix_0[q * kcap + i] = (unsigned short)xi;
     }
@@ -605,7 +608,7 @@ __global__ void __launch_bounds__(kThreads, Y <= 64 ? 3 : 2) fast_adj_kernel(con
     half = true;
   }
   const int hlo = hbuild ? kyo[hb] : 0, hhi = hbuild ? kyo[hb + 1] : 0;
-  const int start = (hr0 / P::START_ROWS) * kcap;
+  const int start = kcap * (NSPLIT == 0 ? hr0 / RP : half ? 1 + hr0 / P::RH : 0);
 
   // coil c's samples into buffer c & 1
   auto issue = [&](int c) {
@@ -630,26 +633,22 @@ __global__ void __launch_bounds__(kThreads, Y <= 64 ? 3 : 2) fast_adj_kernel(con
     const float2* K = Kb + (c & 1) * kcap;
     const float2* ms = A.mps + ((i64)z * A.C + c) * plane + (i64)x * Y + j;
     if (hbuild) {
-      // H[x][ky] += K exp(+2 pi i kx x / X): the term itself steps by conj(W^kx) per row
-      float2 h[RP];
-#pragma unroll
-      for (int r = 0; r < RP; r++) h[r] = make_float2(0.f, 0.f);
+      // H[x][ky] += K exp(+2 pi i kx x / X)
       auto walk = [&](auto rows) {
-        constexpr int ROWS = decltype(rows)::value;
-        for (int i = hlo; i < hhi; i++) {
-          const float2 st = P::TABULATE ? tw_s[i] : cconj(twX[ix_s[i]]);
-          float2 v = cmul(K[i], P::TABULATE ? tw_0[start + i] : cconj(twX[ix_0[start + i]]));
-#pragma unroll
-          for (int r = 0; r < ROWS; r++) {
-            h[r] = cadd(h[r], v);
-            v = cmul(v, st);
-          }
-        }
-#pragma unroll
-        for (int r = 0; r < ROWS; r++) lines[(hr0 + r) * LS + hb] = h[r];
+        h_rows<decltype(rows)::value>(
+            hlo, hhi,
+            [&](int i, float2& v, float2& st) {
+              st = P::TABULATE ? tw_s[i] : cconj(twX[ix_s[i]]);
+              v = cmul(K[i], P::TABULATE ? tw_0[start + i] : cconj(twX[ix_0[start + i]]));
+            },
+            [&](int r, float2 h) { lines[(hr0 + r) * LS + hb] = h; });
       };
-      if (NSPLIT > 0 && half) walk(std::integral_constant<int, P::RH>{});
-      else walk(std::integral_constant<int, RP>{});
+      if constexpr (NSPLIT > 0) {
+        if (half) walk(std::integral_constant<int, P::RH>{});
+        else walk(std::integral_constant<int, RP>{});
+      } else {
+        walk(std::integral_constant<int, RP>{});
+      }
     }
     __syncthreads();
     F::inverse(slots, j, [&](int q, int, float2 v) {

@@ -77,6 +77,45 @@ __device__ __forceinline__ int mulmod(int a, int b, int n, float inv_n) {
   return r;
 }
 
+// The H values of ROWS consecutive rows of one ky bin, H[x] = sum_i v_i st_i^(x - c): sample i's
+// value v at the middle row c = ROWS / 2 and its step st per row come from sample(i, v, st).  Rows
+// c + d and c - d take v st^d and v conj(st^d), which share their four products, so these are
+// accumulated as products and combined once at the end: with the powers of st 4 instructions a
+// row and sample where stepping v itself row by row takes 6 (and half as many steps in the chain).
+// put(r, h) receives row r.
+template <int ROWS, class Sample, class Put>
+__device__ __forceinline__ void h_rows(int lo, int hi, Sample sample, Put put) {
+  constexpr int M = ROWS / 2;
+  static_assert(ROWS >= 2 && ROWS % 2 == 0, "rows pair up around the middle");
+  float2 h0 = make_float2(0.f, 0.f), hm = make_float2(0.f, 0.f);
+  float a[M + 1], b[M + 1], c[M + 1], d[M + 1];  // sums of v.x w.x, v.y w.y, v.x w.y, v.y w.x at distance 1 .. M - 1
+#pragma unroll
+  for (int k = 1; k < M; k++) a[k] = b[k] = c[k] = d[k] = 0.f;
+  for (int i = lo; i < hi; i++) {
+    float2 v, st;
+    sample(i, v, st);
+    float2 w = st;
+    h0 = cadd(h0, v);
+#pragma unroll
+    for (int k = 1; k < M; k++) {
+      a[k] = fmaf(v.x, w.x, a[k]);
+      b[k] = fmaf(v.y, w.y, b[k]);
+      c[k] = fmaf(v.x, w.y, c[k]);
+      d[k] = fmaf(v.y, w.x, d[k]);
+      w = cmul(w, st);
+    }
+    hm.x = fmaf(v.x, w.x, fmaf(v.y, w.y, hm.x));
+    hm.y = fmaf(v.y, w.x, fmaf(-v.x, w.y, hm.y));
+  }
+  put(0, hm);
+  put(M, h0);
+#pragma unroll
+  for (int k = 1; k < M; k++) {
+    put(M + k, make_float2(a[k] - b[k], c[k] + d[k]));
+    put(M - k, make_float2(a[k] + b[k], d[k] - c[k]));
+  }
+}
+
 // The kernels on the run-time two-stage FFT (rt_sense.cu); -1 when ny has no such plan or the
 // mode is not theirs (FWD_LM).
 int try_rt_fwd(FwdArgs& A, int mode, int maxps, int nb, cudaStream_t st);
