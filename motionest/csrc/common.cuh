@@ -59,9 +59,12 @@ __host__ __device__ __forceinline__ float2 mul_mi(float2 a) { return make_float2
 // r^10: truncation below 2e-9).  Rounding the remainder rather than an angle of up to pi to
 // float keeps the phase to 3e-8 (an angle near pi carries 1.2e-7), and nothing branches.
 __device__ __forceinline__ float2 expi_reduced(double phi) {
-  const double t = phi * (4.0 * kInvTwoPi);
-  const double q = rint(t);
-  const float r = (float)((t - q) * (0.25 * kTwoPi));
+  // adding 1.5 2^52 rounds to an integer and leaves its low bits in the sum's low word
+  constexpr double kRound = 6755399441055744.0;
+  const double t = fma(phi, 4.0 * kInvTwoPi, kRound);
+  const int k = __double2loint(t);
+  float r = (float)(fma(phi, 4.0 * kInvTwoPi, kRound - t) * (0.25 * kTwoPi));
+  if (!(fabsf(r) <= 1.0f)) r *= 0.0f;  // NaN and infinity stay NaN; |phi| > 1e15 has no phase
   const float r2 = r * r;
   const float ps = fmaf(r2, fmaf(r2, fmaf(r2, (float)(1.0 / 362880.0), (float)(-1.0 / 5040.0)),
                                  (float)(1.0 / 120.0)), (float)(-1.0 / 6.0));
@@ -69,7 +72,6 @@ __device__ __forceinline__ float2 expi_reduced(double phi) {
                                                    (float)(1.0 / 40320.0)),
                                           (float)(-1.0 / 720.0)), (float)(1.0 / 24.0)), -0.5f);
   const float s = fmaf(r * r2, ps, r), c = fmaf(r2, pc, 1.0f);
-  const int k = (int)(long long)q;
   const float cx = (k & 1) ? s : c, sx = (k & 1) ? c : s;
   return make_float2(((k + 1) & 2) ? -cx : cx, (k & 2) ? -sx : sx);
 }

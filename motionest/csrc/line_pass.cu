@@ -339,6 +339,7 @@ __global__ void __launch_bounds__(pass_threads(N), pass_min_ctas(N, MODE != PM_S
   // the swizzle pattern repeats every 1024 bytes of shared-memory address
   unsigned char* tiles = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   __shared__ __align__(8) uint64_t full[NBUF];
+  __shared__ int4 place_s[NBUF];  // volume, u, v0 and lines of the tile in each buffer
   __shared__ PhaseCoef coef_s[2];
 
   const int tiles_per_vol = STRIDED ? T.row_tiles * A.dims[A.au] : (A.nlines + kTileLines - 1) / kTileLines;
@@ -364,8 +365,10 @@ __global__ void __launch_bounds__(pass_threads(N), pass_min_ctas(N, MODE != PM_S
     bulk_wait_read_all();
     fence_proxy_async_smem();
     __syncwarp();
-    if (threadIdx.x == 0)
+    if (threadIdx.x == 0) {
+      place_s[bufi] = make_int4(vol, u, v0, nl);  // released with the arrival
       mbar_arrive_expect_tx(&full[bufi], NIN * (STRIDED ? TILE : nl * N * 8));
+    }
     __syncwarp();
 #pragma unroll
     for (int k = 0; k < NIN; k++) {
@@ -385,20 +388,20 @@ __global__ void __launch_bounds__(pass_threads(N), pass_min_ctas(N, MODE != PM_S
 
   const bool mover = threadIdx.x < 32;
   if (mover && (int)blockIdx.x < total) issue(blockIdx.x, 0);
+  __syncthreads();  // a wait that gives up must still find the tile's place
   int coef_vol = -1;
   int it = 0;
   for (int t = blockIdx.x; t < total; t += gridDim.x, it++) {
     const int cur = (NBUF == 2) ? (it & 1) : 0;
     const unsigned parity = (NBUF == 2) ? ((it >> 1) & 1) : (it & 1);
-    const int vol = A.div_tiles.div(t);
-    int u, v0, nl;
-    tile_coords<STRIDED>(A, T.div_row, T.row_tiles, t - vol * tiles_per_vol, u, v0, nl);
     mbar_wait_bounded(&full[cur], parity, WF_LINE_PASS);
+    const int4 place = place_s[cur];
+    const int vol = place.x, u = place.y, v0 = place.z, nl = place.w;
     if (NBUF == 2 && mover && t + (int)gridDim.x < total) issue(t + gridDim.x, cur ^ 1);
     // (the barrier before the previous tile's store separates every read of coef_s from a write)
     set_coefs<kDual>(A, vol, coef_vol, coef_s);
     int ul = u, vl = v0 + min(g, nl - 1);
-    if (!STRIDED) {
+    if (!STRIDED && v0 + kTileLines > A.dims[A.av]) {  // the tile runs over into the next rows
       const int l = u * A.dims[A.av] + vl;
       ul = A.div_av.div(l);
       vl = l - ul * A.dims[A.av];
@@ -810,6 +813,8 @@ __global__ void __launch_bounds__(pass_threads(N), pass_min_ctas(N, false))
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char* tiles = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   __shared__ __align__(8) uint64_t full[2];
+  __shared__ int4 place_s[2];  // volume, u, v0 and lines of the tile in each buffer
+  __shared__ int job_s[2];
   __shared__ PhaseCoef coef_s[2];
   const int total = M.tile_off[M.njobs];
   int g, j;
@@ -846,7 +851,11 @@ __global__ void __launch_bounds__(pass_threads(N), pass_min_ctas(N, false))
     bulk_wait_read_all();
     fence_proxy_async_smem();
     __syncwarp();
-    if (threadIdx.x == 0) mbar_arrive_expect_tx(&full[bufi], STRIDED ? TILE : nl * N * 8);
+    if (threadIdx.x == 0) {
+      place_s[bufi] = make_int4(vol, u, v0, nl);  // released with the arrival
+      job_s[bufi] = k;
+      mbar_arrive_expect_tx(&full[bufi], STRIDED ? TILE : nl * N * 8);
+    }
     __syncwarp();
     unsigned char* dst = tiles + bufi * TILE;
     if (STRIDED) {
@@ -862,22 +871,23 @@ __global__ void __launch_bounds__(pass_threads(N), pass_min_ctas(N, false))
 
   const bool mover = threadIdx.x < 32;
   if (mover && (int)blockIdx.x < total) issue(blockIdx.x, 0);
+  __syncthreads();  // a wait that gives up must still find the tile's place
   int coef_job = -1, coef_vol = -1;
   int it = 0;
   for (int t = blockIdx.x; t < total; t += gridDim.x, it++) {
     const int cur = it & 1;
-    const int k = job_of(t);
+    mbar_wait_bounded(&full[cur], (it >> 1) & 1, WF_LINE_PASS);
+    const int4 place = place_s[cur];
+    const int vol = place.x, u = place.y, v0 = place.z, nl = place.w;
+    const int k = job_s[cur];
     const PassArgs& A = M.job[k];
     const MultiTmaJob& J = M.tm[k];
-    int vol, u, v0, nl;
-    coords(k, t, vol, u, v0, nl);
-    mbar_wait_bounded(&full[cur], (it >> 1) & 1, WF_LINE_PASS);
     if (mover && t + (int)gridDim.x < total) issue(t + gridDim.x, cur ^ 1);
     if (k != coef_job) coef_vol = -1;
     coef_job = k;
     set_coefs<false>(A, vol, coef_vol, coef_s);
     int ul = u, vl = v0 + min(g, nl - 1);
-    if (!STRIDED) {
+    if (!STRIDED && v0 + kTileLines > A.dims[A.av]) {  // the tile runs over into the next rows
       const int l = u * A.dims[A.av] + vl;
       ul = A.div_av.div(l);
       vl = l - ul * A.dims[A.av];
