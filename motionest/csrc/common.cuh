@@ -249,6 +249,41 @@ inline cudaError_t allow_smem(K kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// Programmatic dependent launch: a kernel launched by launch_chained may start while the one before
+// it on the stream drains.  It calls chain_wait before its first access to global memory (that
+// returns once the earlier kernels are complete and their writes visible) and chain_next at once,
+// so that its own successor may be set up: the hardware starts that one only when all CTAs of
+// this kernel have started, so no CTA is kept waiting for room.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// `chain`: whether to use it.  Ten dependent passes over one small volume are mostly launch gaps
+// (64x64x48: 83 -> 70 us a transform); a pass whose CTAs each take several tiles is slower with
+// it (ten passes over 32 volumes of 128x112x88: 1.71 -> 2.00 ms), so callers ask for it where the
+// grid is one tile a CTA.  Never while a stream is being captured: the body of a conditional graph
+// node takes plain kernel dependencies.
+template <typename... P, typename... Args>
+inline cudaError_t launch_chained(bool chain, void (*kern)(P...), dim3 grid, int threads,
+                                  size_t smem, cudaStream_t stream, const Args&... args) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = (chain && cudaStreamIsCapturing(stream, &cap) == cudaSuccess &&
+                  cap == cudaStreamCaptureStatusNone) ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+  if (e != cudaSuccess) cudaGetLastError();  // reported here: not left for the next launch
+  return e;
+}
+
 // Count of kernel launches issued by the library (reported by me_launch_count).
 void count_launch();
 void count_launches(long long n);  // n kernels of a graph launch

@@ -240,6 +240,8 @@ __global__ void __launch_bounds__(pass_threads(N),
     cp_async_commit();
   };
 
+  chain_next();
+  chain_wait();
   int cur = 0, coef_vol = -1;
   if ((int)blockIdx.x < total) issue(blockIdx.x, 0);
   for (int t = blockIdx.x; t < total; t += gridDim.x) {
@@ -387,6 +389,8 @@ __global__ void __launch_bounds__(pass_threads(N), pass_min_ctas(N, MODE != PM_S
   };
 
   const bool mover = threadIdx.x < 32;
+  chain_next();
+  chain_wait();
   if (mover && (int)blockIdx.x < total) issue(blockIdx.x, 0);
   __syncthreads();  // a wait that gives up must still find the tile's place
   int coef_vol = -1;
@@ -545,8 +549,9 @@ static int launch_tma(PassArgs& A, const PassTma& T, cudaStream_t stream) {
   static std::atomic<int> occ[8];
   const int grid = pass_grid(kern, pass_threads(N), smem, (long long)tiles * A.nvol, occ);
   count_launch();
-  kern<<<grid, pass_threads(N), smem, stream>>>(A, T);
-  return check_cuda(cudaGetLastError(), "tma pass launch");
+  return check_cuda(launch_chained(grid == (long long)tiles * A.nvol, kern, grid, pass_threads(N),
+                                   smem, stream, A, T),
+                    "tma pass launch");
 }
 
 template <int N, int MODE>
@@ -567,8 +572,9 @@ static int launch_fast(PassArgs& A, cudaStream_t stream) {
   static std::atomic<int> occ[8];
   const int grid = pass_grid(kern, pass_threads(N), smem, (long long)tiles * A.nvol, occ);
   count_launch();
-  kern<<<grid, pass_threads(N), smem, stream>>>(A);
-  return check_cuda(cudaGetLastError(), "fast pass launch");
+  return check_cuda(launch_chained(grid == (long long)tiles * A.nvol, kern, grid, pass_threads(N),
+                                   smem, stream, A),
+                    "fast pass launch");
 }
 
 template <int N>

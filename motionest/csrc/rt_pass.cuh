@@ -85,6 +85,8 @@ __global__ void __launch_bounds__(256, (LARGE || MODE == PM_DUAL_IN || MODE == P
   const int rwrap = half > 0 ? (half - 1) / R1 : 0;  // the last row that starts below N/2
   const double odd_h = (N & 1) ? 0.5 : 0.0;
 
+  chain_next();
+  chain_wait();
   int coef_vol = -1;
   for (int t = blockIdx.x; t < total; t += gridDim.x) {
     const int vol = A.div_tiles.div(t);
@@ -327,8 +329,9 @@ static int launch_rt_t(PassArgs& A, const RtPlan& P, cudaStream_t stream) {
   }
   const long long tiles = (long long)((A.nlines + B - 1) / B) * A.nvol;
   count_launch();
-  kern<<<(int)std::min<long long>(tiles, res), threads, smem, stream>>>(A, P);
-  return check_cuda(cudaGetLastError(), "run-time pass launch");
+  return check_cuda(launch_chained(tiles <= res, kern, (int)std::min<long long>(tiles, res), threads,
+                                   smem, stream, A, P),
+                    "run-time pass launch");
 }
 
 template <int MODE>

@@ -47,6 +47,8 @@ __global__ void __launch_bounds__(kThreads, (MPT > 4 || LARGE) ? 2 : 3)
   float2* spec = tab + NR * T.ls;
   rt_init_twiddles(tw, P);
   init_twiddles(twX, X);
+  chain_next();
+  chain_wait();
 
   const int soff = A.shot_off[s];
   const int ns = A.shot_off[s + 1] - soff;
@@ -169,6 +171,8 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int b = blockIdx.x, x0 = blockIdx.y * NR, z = blockIdx.z;
   const int s = A.shot0 + b;
   const int tid = threadIdx.x;
+  chain_next();
+  chain_wait();
   const int soff = A.shot_off[s];
   const int ns = A.shot_off[s + 1] - soff;
   const int kcap = A.XB;      // max samples per shot, rounded up to even
@@ -284,8 +288,8 @@ static int launch_rt_fwd_t(FwdArgs& A, const RtSense& T, int nb, cudaStream_t st
   if (rc != ME_OK) return rc;
   dim3 grid(nb * A.vps, (A.C + T.cg - 1) / T.cg, A.Z);
   count_launch();
-  rt_fwd_kernel<MPT, MODE, LARGE><<<grid, kThreads, smem, st>>>(A, T);
-  return check_cuda(cudaGetLastError(), "rt sense_fwd launch");
+  return check_cuda(launch_chained(true, rt_fwd_kernel<MPT, MODE, LARGE>, grid, kThreads, smem, st, A, T),
+                    "rt sense_fwd launch");
 }
 
 template <int MODE, bool LARGE>
@@ -318,8 +322,8 @@ static int launch_rt_adj(AdjArgs& A, const RtSense& T, int nb, cudaStream_t st) 
   if (rc != ME_OK) return rc;
   dim3 grid(nb, (A.X + T.NR - 1) / T.NR, A.Z);
   count_launch();
-  rt_adj_kernel<LARGE><<<grid, kThreads, smem, st>>>(A, T);
-  return check_cuda(cudaGetLastError(), "rt sense_adj launch");
+  return check_cuda(launch_chained(true, rt_adj_kernel<LARGE>, grid, kThreads, smem, st, A, T),
+                    "rt sense_adj launch");
 }
 
 int try_rt_adj(AdjArgs& A, int maxps, int nb, cudaStream_t st) {

@@ -288,6 +288,8 @@ __global__ void __launch_bounds__(kThreads, sense_min_ctas(Y)) fast_fwd_kernel(c
   float2* lines = sm;  // one line region per thread group
   float2* twX = lines + P::LINES;
   init_twiddles_any(twX, X);
+  chain_next();
+  chain_wait();
 
   const int soff = A.shot_off[s];
   const int ns = A.shot_off[s + 1] - soff;
@@ -552,6 +554,8 @@ __global__ void __launch_bounds__(kThreads, Y <= 64 ? 3 : 2) fast_adj_kernel(con
   using F = typename P::F;
   constexpr int G = P::G, NG = P::NG, LS = P::LS, RP = P::RP, NSPLIT = P::NSPLIT;
   extern __shared__ __align__(16) float2 sm[];
+  chain_next();
+  chain_wait();
   // shots vary fastest: the CTAs of all shots of one (z, row block) share the map rows in L2
   const int b = blockIdx.x, x0 = blockIdx.y * NG, z = blockIdx.z;
   const int s = A.shot0 + b;
@@ -986,8 +990,8 @@ static int launch_fast_fwd_t(FwdArgs& A, int nb, cudaStream_t st) {
   ME_TRY(check_cuda(allow_smem(fast_fwd_kernel<Y, MPT, MODE>, smem), "fwd smem"));
   dim3 grid(nb * A.vps, A.C, A.Z);
   count_launch();
-  fast_fwd_kernel<Y, MPT, MODE><<<grid, kThreads, smem, st>>>(A);
-  return check_cuda(cudaGetLastError(), "fast sense_fwd launch");
+  return check_cuda(launch_chained(true, fast_fwd_kernel<Y, MPT, MODE>, grid, kThreads, smem, st, A),
+                    "fast sense_fwd launch");
 }
 
 template <int Y, int MODE>
@@ -1058,8 +1062,8 @@ static int launch_fast_adj_y(AdjArgs& A, int maxps, int nb, cudaStream_t st) {
   ME_TRY(check_cuda(allow_smem(fast_adj_kernel<Y>, smem), "adj smem"));
   dim3 grid(nb, (A.X + NG - 1) / NG, A.Z);
   count_launch();
-  fast_adj_kernel<Y><<<grid, kThreads, smem, st>>>(A);
-  return check_cuda(cudaGetLastError(), "fast sense_adj launch");
+  return check_cuda(launch_chained(true, fast_adj_kernel<Y>, grid, kThreads, smem, st, A),
+                    "fast sense_adj launch");
 }
 
 static int try_fast_adj(AdjArgs& A, int maxps, int nb, cudaStream_t st) {
