@@ -294,6 +294,12 @@ long long me_lm_gradient_workspace_bytes(const me_sense* pb, int batch);
 int me_lm_gradient(const me_sense* pb, const me_c64* x, int jac_mode, double* grad, int batch,
                    void* work, void* stream);
 
+/* me_lm_gradient and, where gx is not NULL, gx = sum_s T_s^H C^H F^H M_s (F C T_s x - y) (no
+ * support mask): the gradient of 0.5 sum_s ||M_s F C T_s x - y||^2 with respect to conj(x), from
+ * the same forward and adjoint of each shot.  gx must not be x. */
+int me_lm_gradient_image(const me_sense* pb, const me_c64* x, int jac_mode, double* grad,
+                         me_c64* gx, int batch, void* work, void* stream);
+
 /* Geodesic acceleration (the use_ga branch of transform_estimation.py:75-121): per shot s with
  * LM step v_s = t_next - t (the increment the reference calls v = -delta),
  *   rhs[s][p] = -Re<(J(t_s + eps v_s) v_s - J(t_s) v_s) / eps, J_p(t_s)>,

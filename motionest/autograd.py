@@ -12,8 +12,9 @@ torch.autograd.Function.  Backward is hand-written on the same kernels the solve
     recomputed from x and theta by the shared-prefix Jacobian sweep; nothing from the forward
     pass is stored per shot.
   * d loss / d conj(x) (torch's convention for a complex leaf: the returned gradient is
-    A^H (A x - y)) = sum_s T_s^H C^H F^H M_s F C T_s x - sum_s T_s^H C^H F^H M_s y, the SENSE
-    normal operator and right-hand side without the support mask.
+    A^H (A x - y)) = sum_s T_s^H W_s with W_s = C^H F^H M_s r_s, the volumes that the motion's
+    gradient takes its products with: one adjoint transform more (me_lm_gradient_image).  Without
+    the motion's gradient, one residual pass over the shots without the support mask.
 
 jacobian='exact' (default) gives the true gradient of the loss; jacobian='reference' uses the
 reference's RigidTransformDerivativeCuda convention (the derivative of Tr.Rx.Ry.Rz), which is
@@ -46,15 +47,15 @@ class _ForwardModelLoss(torch.autograd.Function):
         x, t = ctx.saved_tensors
         pb = ctx.pb
         gx = gt = None
+        pb.set_transforms(t)
         if ctx.needs_input_grad[1]:
-            pb.set_transforms(t)
-            grad = pb.lm_gradient(x, ctx.mode)
+            gx = pb.empty_image() if ctx.needs_input_grad[0] else None
+            grad = pb.lm_gradient(x, ctx.mode, image_grad=gx)
             gt = (grad[:, 1:7] * gout).to(ctx.theta_dtype)
-        if ctx.needs_input_grad[0]:
-            pb.set_transforms(t)
-            ax = pb.normal(x, pb.empty_image(), masked=False)
-            b = pb.rhs(pb.empty_image(), masked=False)
-            gx = (ax - b) * gout.to(torch.float32)
+            if gx is not None:
+                gx = gx * gout.to(torch.float32)
+        elif ctx.needs_input_grad[0]:
+            gx = pb.residual(x, pb.empty_image(), masked=False) * -gout.to(torch.float32)
         return gx, gt, None, None
 
 

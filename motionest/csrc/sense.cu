@@ -1494,8 +1494,14 @@ int me_lm_normal_equations(const me_sense* pb, const me_c64* x, int jac_mode, do
 
 int me_lm_gradient(const me_sense* pb, const me_c64* x, int jac_mode, double* grad, int batch,
                    void* work, void* stream) {
+  return me_lm_gradient_image(pb, x, jac_mode, grad, nullptr, batch, work, stream);
+}
+
+int me_lm_gradient_image(const me_sense* pb, const me_c64* x, int jac_mode, double* grad,
+                         me_c64* gx, int batch, void* work, void* stream) {
   ME_TRY(check_problem(pb));
   if (!x || !grad || !work || !pb->ydat) return fail("me_lm_gradient: NULL pointer");
+  if ((const void*)gx == (const void*)x) return fail("me_lm_gradient_image: gx must not be x");
   if (jac_mode != ME_JAC_REFERENCE && jac_mode != ME_JAC_EXACT) return fail("bad jacobian mode");
   cudaStream_t st = (cudaStream_t)stream;
   batch = std::max(1, std::min(batch, pb->nshots));
@@ -1526,6 +1532,14 @@ int me_lm_gradient(const me_sense* pb, const me_c64* x, int jac_mode, double* gr
     count_launch();
     grad_finish_kernel<<<nb, 32, 0, st>>>(w.partial, zc, dpart, nblk, grad, s0);
     ME_TRY(check_cuda(cudaGetLastError(), "gradient finish launch"));
+    if (gx) {
+      // the image's gradient is one adjoint transform away: sum_s T_s^H W_s
+      ME_TRY(R.adjoint(w.U + 7 * vox, bs, w.U + 7 * vox, bs, nb, false));
+      count_launch();
+      sum_volumes_kernel<<<grid_1d(vox), kThreads, 0, st>>>(w.U + 7 * vox, bs, nb, nullptr,
+                                                            (float2*)gx, vox, s0 > 0);
+      ME_TRY(check_cuda(cudaGetLastError(), "sum_volumes launch"));
+    }
   }
   return ME_OK;
 }

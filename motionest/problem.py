@@ -200,12 +200,13 @@ class SenseProblem:
                   _lib.stream_ptr())
         return out
 
-    def residual(self, x, out, energies=None, batch=None):
+    def residual(self, x, out, energies=None, batch=None, masked=True):
         """out = b - A x, the CG's initial residual, from one pass over the shots
         (me_sense_residual); with `energies` ([nshots] float64) also each shot's
         ||M_s (F C T_s x - y)||^2 at the problem's transforms."""
         e = ptr(energies) if energies is not None else None
-        _lib.call("me_sense_residual", self.ref, ptr(x), ptr(out), e, batch or self.batch,
+        ref = self.ref if masked else ctypes.byref(self._unmasked())
+        _lib.call("me_sense_residual", ref, ptr(x), ptr(out), e, batch or self.batch,
                   ptr(self.work), _lib.stream_ptr())
         return out
 
@@ -229,9 +230,10 @@ class SenseProblem:
         _lib.call("me_sense_scatter", self.ref, ptr(K), ptr(ksp_h), _lib.stream_ptr())
         return ksp_h
 
-    def lm_gradient(self, x, jac_mode, out=None, batch=None):
-        """[S, 7] float64: e0 and the gradient g of each shot (me_lm_gradient), with a
-        workspace of its own (the LM workspace, which CG graphs may hold, is left alone)."""
+    def lm_gradient(self, x, jac_mode, out=None, batch=None, image_grad=None):
+        """[S, 7] float64: e0 and the gradient g of each shot (me_lm_gradient); with
+        `image_grad` (a zxy image) also the data term's gradient with respect to conj(x), from
+        the same forward and adjoint of each shot (me_lm_gradient_image).  With a workspace of its own (the LM workspace, which CG graphs may hold, is left alone)."""
         if out is None:
             out = torch.empty((self.nshots, 7), dtype=torch.float64, device=self.device)
         b = batch or self.lm_batch
@@ -240,8 +242,9 @@ class SenseProblem:
             raise ValueError(_lib.load().me_last_error().decode())
         if getattr(self, "_grad_work", None) is None or self._grad_work.numel() < need:
             self._grad_work = torch.empty(int(need), dtype=torch.uint8, device=self.device)
-        _lib.call("me_lm_gradient", self.ref, ptr(x), int(jac_mode), ptr(out), b,
-                  ptr(self._grad_work), _lib.stream_ptr())
+        _lib.call("me_lm_gradient_image", self.ref, ptr(x), int(jac_mode), ptr(out),
+                  ptr(image_grad) if image_grad is not None else None, b, ptr(self._grad_work),
+                  _lib.stream_ptr())
         return out
 
     def lm_stats(self, x, jac_mode, out=None, batch=None):

@@ -118,3 +118,27 @@ def test_gradient_only_statistics_match_full_statistics(jacobian):
     np.testing.assert_allclose(grad[:, 0], full[:, 0], rtol=1e-6)
     scale = np.abs(full[:, 1:7]).max()
     np.testing.assert_allclose(grad[:, 1:7], full[:, 1:7], rtol=1e-4, atol=1e-5 * scale)
+
+
+@pytest.mark.parametrize("batch", [1, 3, 4])
+def test_image_gradient_with_and_without_motion_gradient(batch):
+    """The image gradient that rides on the motion gradient's forward and adjoint (any number of
+    shots per launch), the one residual pass without it, and the FP64 oracle's A x - b."""
+    from motionest.autograd import ForwardModel
+    c = _case()
+    fm = ForwardModel(c["ksp"], c["mps"], c["mask"], c["kg"], c["rk"])
+    fm.pb.set_batches(4, batch)
+    th = torch.tensor(c["t"], device="cuda")
+    grads = []
+    for with_motion in (True, False):
+        x = torch.tensor(c["x"], device="cuda").requires_grad_()
+        t = th.clone().requires_grad_(with_motion)
+        (3.0 * fm.loss(x, t)).backward()
+        assert (t.grad is not None) == with_motion
+        grads.append(x.grad.cpu().numpy())
+    one = np.ones(c["x"].shape)
+    args = (c["mps"].astype(np.complex128), c["mask"], c["t"], c["kg"], c["rk"], one)
+    want = 3.0 * (O64.normal_op(c["x"].astype(np.complex128), *args)
+                  - O64.cg_rhs(c["ksp"].astype(np.complex128), *args))
+    for g in grads:
+        assert np.linalg.norm(g - want) < 2e-5 * np.linalg.norm(want)
