@@ -14,11 +14,14 @@ typedef long long i64;
 constexpr double kTwoPi = 6.283185307179586476925286766559;
 constexpr double kInvTwoPi = 0.15915494309189533576888376337251;
 
+// Products with the roundings written out, so that the same source gives the same bits in
+// every kernel it is inlined into (which of the two products is fused is otherwise the
+// compiler's choice, kernel by kernel).
 __host__ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+  return make_float2(fmaf(a.x, b.x, -(a.y * b.y)), fmaf(a.x, b.y, a.y * b.x));
 }
 __host__ __device__ __forceinline__ float2 cmulc(float2 a, float2 b) {  // a * conj(b)
-  return make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
+  return make_float2(fmaf(a.x, b.x, a.y * b.y), fmaf(a.y, b.x, -(a.x * b.y)));
 }
 __host__ __device__ __forceinline__ float2 cadd(float2 a, float2 b) {
   return make_float2(a.x + b.x, a.y + b.y);
@@ -33,6 +36,10 @@ __host__ __device__ __forceinline__ float2 cconj(float2 a) { return make_float2(
 // a * b + c with four fused multiply-adds
 __host__ __device__ __forceinline__ float2 cfma(float2 a, float2 b, float2 c) {
   return make_float2(fmaf(-a.y, b.y, fmaf(a.x, b.x, c.x)), fmaf(a.y, b.x, fmaf(a.x, b.y, c.y)));
+}
+// a * conj(b) + c
+__host__ __device__ __forceinline__ float2 cfmac(float2 a, float2 b, float2 c) {
+  return make_float2(fmaf(a.y, b.y, fmaf(a.x, b.x, c.x)), fmaf(-a.x, b.y, fmaf(a.y, b.x, c.y)));
 }
 // Division by a divisor 1 <= d < 2^31 fixed at launch, for 0 <= n < 2^31, by the round-up
 // multiply-shift method (Granlund and Montgomery, 1994): q = (umulhi(n, m) + n) >> s with

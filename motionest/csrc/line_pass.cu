@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(pass_threads(N),
     const int u = A.div_av.div(l);
     s0.line = tiles + cur * NT * TILE + g * PITCH;
     s1.line = s0.line + TILE;
-    pass_line<N, MODE>(A, coef_s, u, l - u * dv, j, s0, s1, chirp_s[g]);
+    pass_line<N, MODE>(A, coef_s, u, l - u * dv, j, s0, s1, chirp_s[g], [] {});
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < (MODE == PM_DUAL_OUT ? 2 : 1); k++) {
@@ -401,7 +401,6 @@ __global__ void __launch_bounds__(pass_threads(N), pass_min_ctas(N, MODE != PM_S
     mbar_wait_bounded(&full[cur], parity, WF_LINE_PASS);
     const int4 place = place_s[cur];
     const int vol = place.x, u = place.y, v0 = place.z, nl = place.w;
-    if (NBUF == 2 && mover && t + (int)gridDim.x < total) issue(t + gridDim.x, cur ^ 1);
     // (the barrier before the previous tile's store separates every read of coef_s from a write)
     set_coefs<kDual>(A, vol, coef_vol, coef_s);
     int ul = u, vl = v0 + min(g, nl - 1);
@@ -412,7 +411,12 @@ __global__ void __launch_bounds__(pass_threads(N), pass_min_ctas(N, MODE != PM_S
     }
     s0.line = tiles + cur * NT * TILE + (STRIDED ? 0 : g * PITCH);
     s1.line = s0.line + TILE;
-    pass_line<N, MODE>(A, coef_s, ul, vl, j, s0, s1, chirp_s[g]);
+    // The next tile goes into the buffer that the previous tile is being stored from.  By the end
+    // of the first stage the store has read it; asked for earlier, warp 0 waits for that while
+    // the other warps come to wait for it at the tile's end.
+    pass_line<N, MODE>(A, coef_s, ul, vl, j, s0, s1, chirp_s[g], [&] {
+      if (NBUF == 2 && mover && t + (int)gridDim.x < total) issue(t + gridDim.x, cur ^ 1);
+    });
     // the tile's generic-proxy writes are ordered before the async-proxy store
     fence_proxy_async_smem();
     __syncthreads();
@@ -779,7 +783,7 @@ __global__ void __launch_bounds__(pass_threads(N), pass_min_ctas(N, false))
     const int l = I.l0 + min(g, I.nl - 1);
     const int u = A.div_av.div(l);
     s0.line = tiles + cur * TILE + g * PITCH;
-    pass_line<N, PM_SHEAR>(A, coef_s, u, l - u * A.dims[A.av], j, s0, s0, chirp_s[g]);
+    pass_line<N, PM_SHEAR>(A, coef_s, u, l - u * A.dims[A.av], j, s0, s0, chirp_s[g], [] {});
     __syncthreads();
     if (I.cb < I.nl) {
       const i64 sa = A.st[A.ax];
@@ -888,7 +892,6 @@ __global__ void __launch_bounds__(pass_threads(N), pass_min_ctas(N, false))
     const int k = job_s[cur];
     const PassArgs& A = M.job[k];
     const MultiTmaJob& J = M.tm[k];
-    if (mover && t + (int)gridDim.x < total) issue(t + gridDim.x, cur ^ 1);
     if (k != coef_job) coef_vol = -1;
     coef_job = k;
     set_coefs<false>(A, vol, coef_vol, coef_s);
@@ -900,7 +903,9 @@ __global__ void __launch_bounds__(pass_threads(N), pass_min_ctas(N, false))
     }
     unsigned char* tb = tiles + cur * TILE;
     s0.line = tb + (STRIDED ? 0 : g * PITCH);
-    pass_line<N, PM_SHEAR>(A, coef_s, ul, vl, j, s0, s0, chirp_s[g]);
+    pass_line<N, PM_SHEAR>(A, coef_s, ul, vl, j, s0, s0, chirp_s[g], [&] {
+      if (mover && t + (int)gridDim.x < total) issue(t + gridDim.x, cur ^ 1);
+    });
     fence_proxy_async_smem();
     __syncthreads();
     if (mover) {

@@ -59,10 +59,11 @@ struct LineChirp {
 // The whole of one line (u, v along axes au and av) of pass A in mode MODE by thread j of its
 // G, with the volume's coefficients in coef: s0 and s1 are the line's slots in the first and
 // the second tile (the other input or output of the dual modes), table the line's 2 G chirp
-// table entries.
-template <int N, int MODE, class S>
+// table entries.  midway() is called by every thread after the first stage.
+template <int N, int MODE, class S, class Hook>
 __device__ __forceinline__ void pass_line(const PassArgs& A, const PhaseCoef* coef, int u, int v,
-                                          int j, const S& s0, const S& s1, float2* table) {
+                                          int j, const S& s0, const S& s1, float2* table,
+                                          Hook midway) {
   using L = LineFft<N>;
   constexpr int G = L::G, R1 = L::R1, NI = L::NI;
   constexpr bool kDual = (MODE == PM_DUAL_IN || MODE == PM_DUAL_OUT);
@@ -79,6 +80,7 @@ __device__ __forceinline__ void pass_line(const PassArgs& A, const PhaseCoef* co
   auto store1 = [&](int r, int, float2 x) { s1.tab(r, 0) = x; };
   if (MODE != PM_INV) L::template first<true>(s0, j, load0);
   if (MODE == PM_DUAL_IN) L::template first<true>(s1, j, load1);
+  midway();
   // X (index k + R1 r) times the factors of phase 0 or 1, the form decided once per line
   auto factor = [&](const bool id, const bool sep, const LineChirp<N>& ch, const int q, int k,
                     float2 (&X)[G]) {

@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         for (int q = 0; q < R; q++) u[q] = src[q];
         RDft<R, true>::run(u);
 #pragma unroll
-        for (int q = 0; q < R; q++) w[q] = cadd(w[q], cmulc(u[q], ms[q * R2]));
+        for (int q = 0; q < R; q++) w[q] = cfmac(u[q], ms[q * R2], w[q]);
       });
     }
   }

@@ -656,7 +656,7 @@ __global__ void __launch_bounds__(kThreads, Y <= 64 ? 3 : 2) fast_adj_kernel(con
     }
     __syncthreads();
     F::inverse(slots, j, [&](int q, int, float2 v) {
-      if (live) w[q] = cadd(w[q], cmulc(v, __ldg(ms + q * G)));
+      if (live) w[q] = cfmac(v, __ldg(ms + q * G), w[q]);
     });
   }
   if (live) {
