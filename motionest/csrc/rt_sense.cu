@@ -6,10 +6,11 @@
 // use them (they sit in L2: shots are fastest in the grid), and take a coil at a time, the
 // sample twiddles set up once for all of the CTA's coils.
 //
-// Measured at 160x150x126, 16 coils, 20 shots of 1,200 samples: forward 6.9 ms and adjoint 7.6 ms
+// Measured at 160x150x126, 16 coils, 20 shots of 1,200 samples: forward 6.5 ms and adjoint 6.6 ms
 // where the Stockham kernels of sense.cu took about 96 ms together; the whole normal operator
-// 163.7 -> 23.2 ms.  Widths with a compile-time plan keep their kernels: at 256x224x176, 32 coils,
-// 64 shots these take 67.8 and 90.7 ms, those 55.8 and 63.6 ms.
+// 163.7 -> 21.6 ms.  Reading the sample steps in sample order rather than out of twX took 0.3 and
+// 0.5 ms of that.  Widths with a compile-time plan keep their kernels: at 256x224x176, 32 coils,
+// 64 shots these took 67.8 and 90.7 ms when those took 55.8 and 63.6 ms.
 #include <algorithm>
 
 #include "fft_rt.cuh"
@@ -45,6 +46,10 @@ __global__ void __launch_bounds__(kThreads, (MPT > 4 || LARGE) ? 2 : 3)
   float2* twX = tw + Y;
   float2* tab = twX + X;
   float2* spec = tab + NR * T.ls;
+  // W^kx and W^2kx of each sample: in sample order, where a warp's reads are free of the bank
+  // conflicts of reading them out of twX in every chunk
+  float2* hst = spec + NR * T.ys;
+  float2* hst2 = hst + MPT * kThreads;
   rt_init_twiddles(tw, P);
   init_twiddles(twX, X);
   chain_next();
@@ -52,17 +57,19 @@ __global__ void __launch_bounds__(kThreads, (MPT > 4 || LARGE) ? 2 : 3)
 
   const int soff = A.shot_off[s];
   const int ns = A.shot_off[s + 1] - soff;
-  // per sample: kx, ky, and the step kx NR mod X of its chunk twiddle's index
-  int mkx[MPT], mky[MPT], dix[MPT];
+  __syncthreads();
+  // per sample: ky, and the step kx NR mod X of its chunk twiddle's index
+  int mky[MPT], dix[MPT];
 #pragma unroll
   for (int m = 0; m < MPT; m++) {
     const int jj = tid + m * kThreads;
-    mkx[m] = -1;
     mky[m] = dix[m] = 0;
     if (jj < ns) {
-      mkx[m] = A.kx[soff + jj];
+      const int kx = A.kx[soff + jj];
       mky[m] = A.ky[soff + jj];
-      dix[m] = mulmod(mkx[m], NR % X, X, 1.0f / (float)X);
+      dix[m] = mulmod(kx, NR % X, X, 1.0f / (float)X);
+      hst[jj] = twX[kx];
+      hst2[jj] = twX[2 * kx >= X ? 2 * kx - X : 2 * kx];
     }
   }
   const int g1 = P.d2.div(tid), j1 = tid - g1 * R2;
@@ -70,7 +77,6 @@ __global__ void __launch_bounds__(kThreads, (MPT > 4 || LARGE) ? 2 : 3)
   const bool has1 = g1 < NR, has2 = g2 < NR;
   const i64 plane = (i64)X * Y;
   const float2* vbase = A.vols + (i64)bx * A.vol_stride + (i64)z * plane;
-  __syncthreads();
 
   const int c1 = min(A.C, ((int)blockIdx.y + 1) * T.cg);
   for (int c = blockIdx.y * T.cg; c < c1; c++) {
@@ -118,12 +124,10 @@ __global__ void __launch_bounds__(kThreads, (MPT > 4 || LARGE) ? 2 : 3)
       // (rows past X hold zeros)
 #pragma unroll
       for (int m = 0; m < MPT; m++) {
-        if (mkx[m] < 0) continue;
-        const float2 st = twX[mkx[m]];
+        const int jj = tid + m * kThreads;
+        if (jj >= ns) continue;
+        const float2 st = hst[jj], st2 = hst2[jj];
         const float2 w0 = twX[idx[m]];
-        int kk = 2 * mkx[m];
-        if (kk >= X) kk -= X;
-        const float2 st2 = twX[kk];
         const float2* Lk = spec + mky[m];
         float2 he = Lk[(NR - 2) * T.ys], ho = Lk[(NR - 1) * T.ys];
 #pragma unroll 3
@@ -182,16 +186,18 @@ __global__ void __launch_bounds__(kThreads, 2)
   float2* Kb = twX + X;       // 2 x kcap samples
   float2* H = Kb + 2 * kcap;  // [NR][ys]
   float2* tab = H + NR * T.ys;
-  unsigned short* skx = (unsigned short*)(tab + NR * T.ls);  // kx of a sample, and the index
-  unsigned short* sst = skx + kcap;                          // kx x mod X at each octet's middle
+  float2* tw_s = tab + NR * T.ls;  // conj W^kx of a sample, and conj W^(kx x) at each octet's
+  float2* tw_0 = tw_s + kcap;      // middle
   rt_init_twiddles(tw, P);
   init_twiddles(twX, X);
   const float inv_x = 1.0f / (float)X;
+  __syncthreads();
   for (int i = tid; i < ns; i += kThreads) {
     const int kx = A.kx[soff + i];
-    skx[i] = (unsigned short)kx;
+    tw_s[i] = cconj(twX[kx]);
     for (int o = 0; o < no; o++)
-      sst[o * kcap + i] = (unsigned short)mulmod(kx, (x0 + o * kOctet + kOctet / 2) % X, X, inv_x);
+      tw_0[o * kcap + i] =
+          cconj(twX[mulmod(kx, (x0 + o * kOctet + kOctet / 2) % X, X, inv_x)]);
   }
   const int* kyo = A.ky_off + (i64)s * (Y + 1);
   const int* order = A.ky_order ? A.ky_order + (i64)s * Y : nullptr;
@@ -225,8 +231,8 @@ __global__ void __launch_bounds__(kThreads, 2)
       h_rows<kOctet>(
           kyo[bin], kyo[bin + 1],
           [&](int i, float2& v, float2& st) {
-            st = cconj(twX[skx[i]]);
-            v = cmulc(K[i], twX[sst[o * kcap + i]]);
+            st = tw_s[i];
+            v = cmul(K[i], tw_0[o * kcap + i]);
           },
           [&](int r, float2 h) { H[(o * kOctet + r) * T.ys + bin] = h; });
     }
@@ -283,7 +289,8 @@ bool has_rt_sense(int ny) {
 
 template <int MPT, int MODE, bool LARGE>
 static int launch_rt_fwd_t(FwdArgs& A, const RtSense& T, int nb, cudaStream_t st) {
-  const size_t smem = sizeof(float2) * ((size_t)A.Y + A.X + (size_t)T.NR * (T.ls + T.ys));
+  const size_t smem = sizeof(float2) * ((size_t)A.Y + A.X + (size_t)T.NR * (T.ls + T.ys) +
+                                        2 * MPT * (size_t)kThreads);
   const int rc = check_cuda(allow_smem(rt_fwd_kernel<MPT, MODE, LARGE>, smem), "rt fwd smem");
   if (rc != ME_OK) return rc;
   dim3 grid(nb * A.vps, (A.C + T.cg - 1) / T.cg, A.Z);
@@ -315,9 +322,8 @@ int try_rt_fwd(FwdArgs& A, int mode, int maxps, int nb, cudaStream_t st) {
 
 template <bool LARGE>
 static int launch_rt_adj(AdjArgs& A, const RtSense& T, int nb, cudaStream_t st) {
-  const size_t smem = sizeof(float2) * ((size_t)A.Y + A.X + 2 * (size_t)A.XB +
-                                        (size_t)T.NR * (T.ls + T.ys)) +
-                      sizeof(unsigned short) * (size_t)A.XB * (1 + T.NR / kOctet);
+  const size_t smem = sizeof(float2) * ((size_t)A.Y + A.X + (3 + T.NR / kOctet) * (size_t)A.XB +
+                                        (size_t)T.NR * (T.ls + T.ys));
   const int rc = check_cuda(allow_smem(rt_adj_kernel<LARGE>, smem), "rt adj smem");
   if (rc != ME_OK) return rc;
   dim3 grid(nb, (A.X + T.NR - 1) / T.NR, A.Z);
