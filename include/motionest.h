@@ -99,8 +99,8 @@ long long me_launch_count(void);
  * and lets the kernel finish, so a lost copy ends as an error instead of a hung GPU.  No
  * counterpart in the reference (CuPy and cuFFT have no such waits).
  * me_wait_status synchronises the current device, returns the OR of the recorded bits in
- * *status (0: no wait ran out; 1 SENSE forward, 2 SENSE adjoint, 4 line pass, 0x100 the
- * self-test) and clears them.  Results of launches before a non-zero status are not to be
+ * *status (0: no wait ran out; 4 line pass, 0x100 the self-test; 1 and 2, the SENSE kernels, no
+ * longer occur: these stage nothing) and clears them.  Results of launches before a non-zero status are not to be
  * trusted.  me_wait_selftest launches one CTA whose barrier never completes (one arrival short
  * of its count) and whose wait gives up after limit_cycles (1 .. 2^31) clock cycles; the next
  * me_wait_status then reports 0x100. */

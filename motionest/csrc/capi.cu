@@ -26,7 +26,6 @@ int check_cuda(cudaError_t e, const char* what) {
   return ME_ERR_CUDA;
 }
 
-int sense_wait_fault(unsigned* out);
 int line_pass_wait_fault(unsigned* out);
 ME_WAIT_FAULT_ACCESSOR(capi_wait_fault)
 
@@ -63,11 +62,10 @@ long long me_launch_count(void) { return g_launches.load(std::memory_order_relax
 
 int me_wait_status(unsigned* status) {
   if (!status) return fail("me_wait_status: NULL pointer");
-  unsigned a = 0, b = 0, c = 0;
-  ME_CHECK_RC(sense_wait_fault(&a));
-  ME_CHECK_RC(line_pass_wait_fault(&b));
-  ME_CHECK_RC(capi_wait_fault(&c));
-  *status = a | b | c;
+  unsigned a = 0, b = 0;
+  ME_CHECK_RC(line_pass_wait_fault(&a));
+  ME_CHECK_RC(capi_wait_fault(&b));
+  *status = a | b;
   return ME_OK;
 }
 

@@ -242,8 +242,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity
 
 // Fault codes recorded by the bounded waits (bits, OR-ed together).
 enum WaitFault : unsigned {
-  WF_SENSE_FWD = 1u,
-  WF_SENSE_ADJ = 2u,
   WF_LINE_PASS = 4u,
   WF_SELFTEST = 0x100u,
 };

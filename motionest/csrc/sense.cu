@@ -970,8 +970,6 @@ static int launch_fwd_v(FwdArgs& A, int maxps, int nb, cudaStream_t st) {
   return launch_fwd_t<8, V, MODE>(A, nb, st);
 }
 
-ME_WAIT_FAULT_ACCESSOR(sense_wait_fault)
-
 // The LM statistics from the fused seven-volume kernel unless ME_LM_TWO_PASS=1 (the forward
 // kernel writing seven K regions, then lm_stats_kernel; bit-identical, kept for comparison).
 static bool fused_lm_enabled() {
