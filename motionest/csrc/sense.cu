@@ -1012,11 +1012,17 @@ static int launch_fast_lm_t(FwdArgs& A, int nb, cudaStream_t st) {
 }
 
 // The fused statistics kernel keeps seven accumulators per sample in registers: up to two
-// samples per thread (512 per shot); more take the two-kernel path.
+// samples per thread (512 per shot).  It serves widths up to 128 points (64x64x48, 8 coils, 16
+// shots: 1.64 ms a statistics call against 1.72 in two kernels; 128x128x96, 16 coils, 32 shots:
+// 28.3 against 29.1).  Above, the forward kernel, which has the registers to keep its sample
+// twiddles, is faster seven times over than the fused kernel (256x224x32, 32 coils, 64 shots:
+// 102.3 ms against 103.9).
 template <int Y>
 static int launch_fast_lm_y(FwdArgs& A, int maxps, int nb, cudaStream_t st) {
-  if (maxps <= kThreads) return launch_fast_lm_t<Y, 1>(A, nb, st);
-  if (maxps <= 2 * kThreads) return launch_fast_lm_t<Y, 2>(A, nb, st);
+  if constexpr (line_threads(Y) == 8) {
+    if (maxps <= kThreads) return launch_fast_lm_t<Y, 1>(A, nb, st);
+    if (maxps <= 2 * kThreads) return launch_fast_lm_t<Y, 2>(A, nb, st);
+  }
   return -1;
 }
 
