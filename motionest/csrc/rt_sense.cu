@@ -6,9 +6,9 @@
 // use them (they sit in L2: shots are fastest in the grid), and take a coil at a time, the
 // sample twiddles set up once for all of the CTA's coils.
 //
-// Measured at 160x150x126, 16 coils, 20 shots of 1,200 samples: forward 6.5 ms and adjoint 6.6 ms
+// Measured at 160x150x126, 16 coils, 20 shots of 1,200 samples: forward 6.3 ms and adjoint 6.6 ms
 // where the Stockham kernels of sense.cu took about 96 ms together; the whole normal operator
-// 163.7 -> 21.6 ms.  Reading the sample steps in sample order rather than out of twX took 0.3 and
+// 163.7 -> 21.4 ms.  Reading the sample steps in sample order rather than out of twX took 0.3 and
 // 0.5 ms of that.  Widths with a compile-time plan keep their kernels: at 256x224x176, 32 coils,
 // 64 shots these took 67.8 and 90.7 ms when those took 55.8 and 63.6 ms.
 #include <algorithm>
@@ -46,10 +46,11 @@ __global__ void __launch_bounds__(kThreads, (MPT > 4 || LARGE) ? 2 : 3)
   float2* twX = tw + Y;
   float2* tab = twX + X;
   float2* spec = tab + NR * T.ls;
-  // W^kx and W^2kx of each sample: in sample order, where a warp's reads are free of the bank
+  // W^kx, W^2kx and W^4kx of each sample: in sample order, where a warp's reads are free of the bank
   // conflicts of reading them out of twX in every chunk
   float2* hst = spec + NR * T.ys;
   float2* hst2 = hst + MPT * kThreads;
+  float2* hst4 = hst2 + MPT * kThreads;
   rt_init_twiddles(tw, P);
   init_twiddles(twX, X);
   chain_next();
@@ -69,7 +70,8 @@ __global__ void __launch_bounds__(kThreads, (MPT > 4 || LARGE) ? 2 : 3)
       mky[m] = A.ky[soff + jj];
       dix[m] = mulmod(kx, NR % X, X, 1.0f / (float)X);
       hst[jj] = twX[kx];
-      hst2[jj] = twX[2 * kx >= X ? 2 * kx - X : 2 * kx];
+      hst2[jj] = twX[2 * kx % X];
+      hst4[jj] = twX[4 * kx % X];
     }
   }
   const int g1 = P.d2.div(tid), j1 = tid - g1 * R2;
@@ -120,22 +122,26 @@ __global__ void __launch_bounds__(kThreads, (MPT > 4 || LARGE) ? 2 : 3)
         });
       }
       __syncthreads();
-      // sample sums over the chunk's rows by Horner's rule in two chains, as fast_fwd_kernel
-      // (rows past X hold zeros)
+      // sample sums over the chunk's rows by Horner's rule in four chains, each stepping by W^4kx
+      // (rows past X hold zeros): a chain of 31 rows would carry the rounding of its step up to
+      // the 15th power
 #pragma unroll
       for (int m = 0; m < MPT; m++) {
         const int jj = tid + m * kThreads;
         if (jj >= ns) continue;
-        const float2 st = hst[jj], st2 = hst2[jj];
+        const float2 st = hst[jj], st2 = hst2[jj], st4 = hst4[jj];
         const float2 w0 = twX[idx[m]];
         const float2* Lk = spec + mky[m];
-        float2 he = Lk[(NR - 2) * T.ys], ho = Lk[(NR - 1) * T.ys];
-#pragma unroll 3
-        for (int i = NR - 4; i >= 0; i -= 2) {
-          he = cfma(he, st2, Lk[i * T.ys]);
-          ho = cfma(ho, st2, Lk[(i + 1) * T.ys]);
+        float2 h[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) h[q] = Lk[(NR - 4 + q) * T.ys];
+#pragma unroll 2
+        for (int i = NR - 8; i >= 0; i -= 4) {
+#pragma unroll
+          for (int q = 0; q < 4; q++) h[q] = cfma(h[q], st4, Lk[(i + q) * T.ys]);
         }
-        acc[m] = cfma(cfma(ho, st, he), w0, acc[m]);
+        const float2 lo = cfma(h[1], st, h[0]), hi = cfma(h[3], st, h[2]);
+        acc[m] = cfma(cfma(hi, st2, lo), w0, acc[m]);
         idx[m] += dix[m];
         if (idx[m] >= X) idx[m] -= X;
       }
@@ -290,7 +296,7 @@ bool has_rt_sense(int ny) {
 template <int MPT, int MODE, bool LARGE>
 static int launch_rt_fwd_t(FwdArgs& A, const RtSense& T, int nb, cudaStream_t st) {
   const size_t smem = sizeof(float2) * ((size_t)A.Y + A.X + (size_t)T.NR * (T.ls + T.ys) +
-                                        2 * MPT * (size_t)kThreads);
+                                        3 * MPT * (size_t)kThreads);
   const int rc = check_cuda(allow_smem(rt_fwd_kernel<MPT, MODE, LARGE>, smem), "rt fwd smem");
   if (rc != ME_OK) return rc;
   dim3 grid(nb * A.vps, (A.C + T.cg - 1) / T.cg, A.Z);
