@@ -271,13 +271,53 @@ struct FwdPlan {
   static constexpr int LINES = NG * LS;
 };
 
+// sum_row L[row] W^(kx row) over a chunk's RC rows of one spectrum column (rows LS apart) by
+// Horner's rule in interleaved chains of eight rows: two stepping by W^2kx, or four by W^4kx where
+// a chunk has 32 rows.  A chain carries the rounding of its step up to its length.  At 128 points, 128
+// rows, against 64 bits: two chains of sixteen 2.53e-7, four of eight 1.77e-7 (two chains over
+// chunks of 16 rows: 1.72e-7); 32 planes, 8 coils, 8 shots of 400 samples 101.9 and 102.8 us, of 1,000
+// samples 147.9 and 155.2 us.  (Two sums of 16 rows a chunk, each with a table twiddle of its own:
+// 1.72e-7, 106.6 and 159.5 us.)
+constexpr int fwd_chains(int rc) { return rc >= 32 ? 4 : 2; }
+template <int RC, int LS>
+__device__ __forceinline__ float2 sample_sum(const float2* Lk, float2 st, float2 st2, float2 st4) {
+  constexpr int NC = fwd_chains(RC);
+  static_assert(RC % NC == 0, "the chains take rows in turn");
+  const float2 step = NC == 4 ? st4 : st2;
+  float2 h[NC];
+#pragma unroll
+  for (int q = 0; q < NC; q++) h[q] = Lk[(RC - NC + q) * LS];
+#pragma unroll
+  for (int i = RC - 2 * NC; i >= 0; i -= NC) {
+#pragma unroll
+    for (int q = 0; q < NC; q++) h[q] = cfma(h[q], step, Lk[(i + q) * LS]);
+  }
+  const float2 lo = cfma(h[1], st, h[0]);
+  if (NC == 2) return lo;
+  return cfma(cfma(h[NC - 1], st, h[NC - 2]), st2, lo);
+}
+
+// The steps W^kx, W^2kx and W^4kx of a sample (the last one where there are four chains).
+struct SampleSteps {
+  float2 st, st2, st4;
+  template <int RC>
+  __device__ __forceinline__ void set(const float2* twX, int kx, int X) {
+    int k = 2 * kx;
+    if (k >= X) k -= X;
+    st = twX[kx];
+    st2 = twX[k];
+    k *= 2;
+    if (k >= X) k -= X;
+    st4 = fwd_chains(RC) == 4 ? twX[k] : st2;
+  }
+};
+
 template <int Y, int MPT, int MODE>
 __global__ void __launch_bounds__(kThreads, sense_min_ctas(Y)) fast_fwd_kernel(const FwdArgs A) {
   static_assert(MODE == FWD_K || MODE == FWD_RESID, "one volume per CTA");
   using P = FwdPlan<Y>;
   using F = typename P::F;
   constexpr int G = P::G, RC = P::RC, LS = P::LS;
-  static_assert(RC % 2 == 0, "the two Horner chains take rows in pairs");
   extern __shared__ __align__(16) float2 sm[];
   // shots vary fastest, so the CTAs of all shots of one (z, coil) run together and share the
   // map plane (and each shot's image plane across coils) through L2
@@ -318,19 +358,14 @@ __global__ void __launch_bounds__(kThreads, sense_min_ctas(Y)) fast_fwd_kernel(c
   PaddedSlots<Y> slots;
   slots.init(lines + g * LS, j);
 
-  // The Horner steps W^kx and W^2kx do not change between chunks: with few samples per thread
-  // they are read from the table once (registers), else once per chunk.
+  // The Horner steps do not change between chunks: with few samples per thread they are read from
+  // the table once (registers), else once per chunk.
   constexpr bool kHoist = MPT <= 2;
-  float2 hst[kHoist ? MPT : 1], hst2[kHoist ? MPT : 1];
+  SampleSteps hst[kHoist ? MPT : 1];
   __syncthreads();  // twX is written above by all threads
   if constexpr (kHoist) {
 #pragma unroll
-    for (int m = 0; m < MPT; m++) {
-      const int kx = mkx[m] < 0 ? 0 : mkx[m];
-      const int k2 = 2 * kx >= X ? 2 * kx - X : 2 * kx;
-      hst[m] = twX[kx];
-      hst2[m] = twX[k2];
-    }
+    for (int m = 0; m < MPT; m++) hst[m].set<RC>(twX, mkx[m] < 0 ? 0 : mkx[m], X);
   }
   for (int x0 = 0; x0 < X; x0 += RC) {
     const int nr = min(RC, X - x0);
@@ -346,26 +381,15 @@ __global__ void __launch_bounds__(kThreads, sense_min_ctas(Y)) fast_fwd_kernel(c
       });
     }
     __syncthreads();
-    // Sample sums over the chunk's rows by Horner's rule, sum_row L[row] W^(kx row), then one
-    // table twiddle W^(kx x0) per chunk.  Rows past nr hold zeros (zero lines transform to
-    // zero), so every chunk runs all RC rows, in two interleaved chains (even and odd rows,
-    // stepping by W^(2 kx)) so that two FMA chains are in flight.
+    // Sample sums over the chunk's rows, then one table twiddle W^(kx x0) per chunk.  Rows past nr
+    // hold zeros (zero lines transform to zero), so every chunk runs all RC rows.
 #pragma unroll
     for (int m = 0; m < MPT; m++) {
       if (mkx[m] < 0) continue;
-      const float2 st = kHoist ? hst[m] : twX[mkx[m]];
-      const float2 w0 = twX[idx[m]];
-      const float2* Lk = lines + mky[m];
-      int k2 = 2 * mkx[m];
-      if (k2 >= X) k2 -= X;
-      const float2 st2 = kHoist ? hst2[m] : twX[k2];
-      float2 he = Lk[(RC - 2) * LS], ho = Lk[(RC - 1) * LS];
-#pragma unroll
-      for (int i = RC / 2 - 2; i >= 0; i--) {
-        he = cfma(he, st2, Lk[(2 * i) * LS]);
-        ho = cfma(ho, st2, Lk[(2 * i + 1) * LS]);
-      }
-      acc[m] = cfma(cfma(ho, st, he), w0, acc[m]);
+      SampleSteps t;
+      if (kHoist) t = hst[m];
+      else t.set<RC>(twX, mkx[m], X);
+      acc[m] = cfma(sample_sum<RC, LS>(lines + mky[m], t.st, t.st2, t.st4), twX[idx[m]], acc[m]);
       idx[m] += dix[m];
       if (idx[m] >= X) idx[m] -= X;
     }
@@ -408,7 +432,6 @@ __global__ void __launch_bounds__(kThreads, 2) fast_lm_kernel(const FwdArgs A) {
   using F = typename P::F;
   constexpr int G = P::G, RC = P::RC, LS = P::LS;
   constexpr int NV = 7;
-  static_assert(RC % 2 == 0, "the two Horner chains take rows in pairs");
   extern __shared__ __align__(16) float2 sm[];
   const int b = blockIdx.x, c = blockIdx.y, z = blockIdx.z;
   const int s = A.shot0 + b;
@@ -445,16 +468,11 @@ __global__ void __launch_bounds__(kThreads, 2) fast_lm_kernel(const FwdArgs A) {
   slots.init(lines + g * LS, j);
 
   constexpr bool kHoist = MPT <= 2;
-  float2 hst[kHoist ? MPT : 1], hst2[kHoist ? MPT : 1];
+  SampleSteps hst[kHoist ? MPT : 1];
   __syncthreads();  // twX is written above by all threads
   if constexpr (kHoist) {
 #pragma unroll
-    for (int m = 0; m < MPT; m++) {
-      const int kx = mkx[m] < 0 ? 0 : mkx[m];
-      const int k2 = 2 * kx >= X ? 2 * kx - X : 2 * kx;
-      hst[m] = twX[kx];
-      hst2[m] = twX[k2];
-    }
+    for (int m = 0; m < MPT; m++) hst[m].set<RC>(twX, mkx[m] < 0 ? 0 : mkx[m], X);
   }
   for (int x0 = 0; x0 < X; x0 += RC) {
     const int nr = min(RC, X - x0);
@@ -474,21 +492,13 @@ __global__ void __launch_bounds__(kThreads, 2) fast_lm_kernel(const FwdArgs A) {
 #pragma unroll
       for (int m = 0; m < MPT; m++) {
         if (mkx[m] < 0) continue;
-        const float2 st = kHoist ? hst[m] : twX[mkx[m]];
-        const float2 w0 = twX[idx[m]];
-        const float2* Lk = lines + mky[m];
-        int k2 = 2 * mkx[m];
-        if (k2 >= X) k2 -= X;
-        const float2 st2 = kHoist ? hst2[m] : twX[k2];
-        float2 he = Lk[(RC - 2) * LS], ho = Lk[(RC - 1) * LS];
-#pragma unroll
-        for (int i = RC / 2 - 2; i >= 0; i--) {
-          he = cfma(he, st2, Lk[(2 * i) * LS]);
-          ho = cfma(ho, st2, Lk[(2 * i + 1) * LS]);
-        }
+        SampleSteps t;
+        if (kHoist) t = hst[m];
+        else t.set<RC>(twX, mkx[m], X);
+        const float2 sum = sample_sum<RC, LS>(lines + mky[m], t.st, t.st2, t.st4);
         // the accumulators rotate as a queue, so that volume v's is always acc[0] (v is not a
         // compile-time index); after the seven volumes of a chunk acc[u] is volume u's again
-        const float2 nv = cfma(cfma(ho, st, he), w0, acc[0][m]);
+        const float2 nv = cfma(sum, twX[idx[m]], acc[0][m]);
 #pragma unroll
         for (int u = 0; u < NV - 1; u++) acc[u][m] = acc[u + 1][m];
         acc[NV - 1][m] = nv;
