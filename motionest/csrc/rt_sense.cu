@@ -189,11 +189,12 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int no = NR / kOctet;
   float2* tw = sm;
   float2* twX = tw + Y;
-  float2* Kb = twX + X;       // 2 x kcap samples
-  float2* H = Kb + 2 * kcap;  // [NR][ys]
+  float2* K = twX + X;        // kcap samples of a coil
+  float2* H = K + kcap;       // [NR][ys]
   float2* tab = H + NR * T.ys;
-  float2* tw_s = tab + NR * T.ls;  // conj W^kx of a sample, and conj W^(kx x) at each octet's
-  float2* tw_0 = tw_s + kcap;      // middle
+  float2* tw_s = tab + NR * T.ls;  // conj W^kx and conj W^3kx of a sample,
+  float2* tw_3 = tw_s + kcap;
+  float2* tw_0 = tw_3 + kcap;      // and conj W^(kx x) at each octet's middle
   rt_init_twiddles(tw, P);
   init_twiddles(twX, X);
   const float inv_x = 1.0f / (float)X;
@@ -201,6 +202,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   for (int i = tid; i < ns; i += kThreads) {
     const int kx = A.kx[soff + i];
     tw_s[i] = cconj(twX[kx]);
+    tw_3[i] = cconj(twX[3 * kx % X]);
     for (int o = 0; o < no; o++)
       tw_0[o * kcap + i] =
           cconj(twX[mulmod(kx, (x0 + o * kOctet + kOctet / 2) % X, X, inv_x)]);
@@ -216,8 +218,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 
   auto issue = [&](int c) {
     const float2* kc = A.kin + kbase0 + ((i64)z * A.C + c) * ns;
-    float2* kd = Kb + (c & 1) * kcap;
-    for (int i = tid; i < ns; i += kThreads) cp_async8(kd + i, kc + i);
+    for (int i = tid; i < ns; i += kThreads) cp_async8(K + i, kc + i);
     cp_async_commit();
   };
   float2 w[kRtMaxR1];
@@ -228,21 +229,21 @@ __global__ void __launch_bounds__(kThreads, 2)
   for (int c = 0; c < A.C; c++) {
     cp_async_wait_all();
     __syncthreads();
-    if (c + 1 < A.C) issue(c + 1);
-    const float2* K = Kb + (c & 1) * kcap;
     // H[x][ky] += K exp(+2 pi i kx x / X), eight rows of one bin per item, heaviest bins first
     for (int q = tid; q < Y * no; q += kThreads) {
       const int slot = q / no, o = q - slot * no;
       const int bin = order ? order[slot] : slot;
-      h_rows<kOctet>(
+      h_rows<kOctet, true>(
           kyo[bin], kyo[bin + 1],
-          [&](int i, float2& v, float2& st) {
+          [&](int i, float2& v, float2& st, float2& st3) {
             st = tw_s[i];
+            st3 = tw_3[i];
             v = cmul(K[i], tw_0[o * kcap + i]);
           },
           [&](int r, float2 h) { H[(o * kOctet + r) * T.ys + bin] = h; });
     }
     __syncthreads();
+    if (c + 1 < A.C) issue(c + 1);  // arrives under the FFT
     if (has2) {
       rt_switch2<LARGE>(R2, [&](auto rc) {
         constexpr int R = decltype(rc)::value;
@@ -267,7 +268,8 @@ __global__ void __launch_bounds__(kThreads, 2)
         for (int q = 0; q < R; q++) u[q] = src[q];
         RDft<R, true>::run(u);
 #pragma unroll
-        for (int q = 0; q < R; q++) w[q] = cfmac(u[q], ms[q * R2], w[q]);
+        for (int q = 0; q < R; q++)  // (one rounding of the sum a coil; fused, two)
+          w[q] = cadd(w[q], cmulc(u[q], ms[q * R2]));
       });
     }
   }

@@ -553,6 +553,12 @@ struct AdjPlan {
   // shared bin); their sample twiddles are tabulated as factors when they are few
   static constexpr int STARTS = NSPLIT > 0 ? 3 : NPARTS;
   static constexpr bool TABULATE = STARTS <= 3;
+  // W^3kx is tabulated too (h_rows) where threads walk all their rows in step
+  static constexpr bool CUBE = TABULATE && NSPLIT == 0 && RP >= 8;
+  // With that table in the place of the second sample buffer, the next coil's samples arrive under
+  // the FFT alone.
+  static constexpr int NK = CUBE ? 1 : 2;
+  static constexpr int TABLES = 1 + STARTS + (CUBE ? 1 : 0);
   static __host__ __device__ constexpr int start_row(int q) {
     return NSPLIT > 0 ? (q == 0 ? RH : q == 1 ? RH / 2 : RH + RH / 2) : q * RP + RP / 2;
   }
@@ -573,14 +579,15 @@ __global__ void __launch_bounds__(kThreads, Y <= 64 ? 3 : 2) fast_adj_kernel(con
   const int soff = A.shot_off[s];
   const int ns = A.shot_off[s + 1] - soff;
   const int kcap = (A.XB + 1) & ~1;   // max samples per shot, padded
-  float2* Kb = sm;                    // 2 x kcap samples
-  float2* lines = Kb + 2 * kcap;      // NG x LS
+  float2* Kb = sm;                    // NK x kcap samples
+  float2* lines = Kb + P::NK * kcap;  // NG x LS
   float2* twX = lines + NG * LS;
   // per sample, shared by all coils: conj W^kx and, at the middle row of each of the P::STARTS row
-  // ranges that threads build, conj W^(kx x) -- as factors, or (short lines, many ranges) as
-  // indices into twX
+  // ranges that threads build, conj W^(kx x) -- as factors (and conj W^3kx where P::CUBE), or
+  // (short lines, many ranges) as indices into twX
   float2* tw_s = twX + pad2(X);
   float2* tw_0 = tw_s + kcap;
+  float2* tw_3 = tw_0 + P::STARTS * kcap;
   unsigned short* ix_s = reinterpret_cast<unsigned short*>(tw_s);
   unsigned short* ix_0 = ix_s + kcap;
   init_twiddles_any(twX, X);
@@ -598,6 +605,7 @@ __global__ void __launch_bounds__(kThreads, Y <= 64 ? 3 : 2) fast_adj_kernel(con
     const int kx = A.kx[soff + i];
     if (P::TABULATE) tw_s[i] = cconj(twX[kx]);
     else ix_s[i] = (unsigned short)kx;
+    if (P::CUBE) tw_3[i] = cconj(twX[3 * kx % X]);
     for (int q = 0; q < P::STARTS; q++) {
       const int xi = mulmod(kx, (x0 + P::start_row(q)) % X, X, inv_x);
       if (P::TABULATE) tw_0[q * kcap + i] = cconj(twX[xi]);
@@ -624,10 +632,10 @@ __global__ void __launch_bounds__(kThreads, Y <= 64 ? 3 : 2) fast_adj_kernel(con
   const int hlo = hbuild ? kyo[hb] : 0, hhi = hbuild ? kyo[hb + 1] : 0;
   const int start = kcap * (NSPLIT == 0 ? hr0 / RP : half ? 1 + hr0 / P::RH : 0);
 
-  // coil c's samples into buffer c & 1
+  // coil c's samples into buffer c mod NK
   auto issue = [&](int c) {
     const float2* kc = A.kin + kbase0 + ((i64)z * A.C + c) * ns;
-    float2* kd = Kb + (c & 1) * kcap;
+    float2* kd = Kb + (c % P::NK) * kcap;
     for (int i = threadIdx.x; i < ns; i += kThreads) cp_async8(kd + i, kc + i);
     cp_async_commit();
   };
@@ -643,16 +651,17 @@ __global__ void __launch_bounds__(kThreads, Y <= 64 ? 3 : 2) fast_adj_kernel(con
   for (int c = 0; c < A.C; c++) {
     cp_async_wait_all();
     __syncthreads();
-    if (c + 1 < A.C) issue(c + 1);
-    const float2* K = Kb + (c & 1) * kcap;
+    if (P::NK == 2 && c + 1 < A.C) issue(c + 1);
+    const float2* K = Kb + (c % P::NK) * kcap;
     const float2* ms = A.mps + ((i64)z * A.C + c) * plane + (i64)x * Y + j;
     if (hbuild) {
       // H[x][ky] += K exp(+2 pi i kx x / X)
       auto walk = [&](auto rows) {
-        h_rows<decltype(rows)::value>(
+        h_rows<decltype(rows)::value, P::CUBE>(
             hlo, hhi,
-            [&](int i, float2& v, float2& st) {
+            [&](int i, float2& v, float2& st, float2& st3) {
               st = P::TABULATE ? tw_s[i] : cconj(twX[ix_s[i]]);
+              if (P::CUBE) st3 = tw_3[i];
               v = cmul(K[i], P::TABULATE ? tw_0[start + i] : cconj(twX[ix_0[start + i]]));
             },
             [&](int r, float2 h) { lines[(hr0 + r) * LS + hb] = h; });
@@ -665,8 +674,14 @@ __global__ void __launch_bounds__(kThreads, Y <= 64 ? 3 : 2) fast_adj_kernel(con
       }
     }
     __syncthreads();
+    if (P::NK == 1 && c + 1 < A.C) issue(c + 1);
+    // Added to the sum over the coils as one term, the product rounds it once; fused into it, twice
+    // (128 points, 32 coils: 1.6e-7 from 64 bits and, fused, 2.1e-7).  Sixteen threads a line keep
+    // the fused form: the other one spills at 192 and 224 points (1.5 to 5% there).
     F::inverse(slots, j, [&](int q, int, float2 v) {
-      if (live) w[q] = cfmac(v, __ldg(ms + q * G), w[q]);
+      if (!live) return;
+      const float2 m = __ldg(ms + q * G);
+      w[q] = G == 8 ? cadd(w[q], cmulc(v, m)) : cfmac(v, m, w[q]);
     });
   }
   if (live) {
@@ -1071,8 +1086,8 @@ static int launch_fast_adj_y(AdjArgs& A, int maxps, int nb, cudaStream_t st) {
   constexpr int NG = P::NG;
   A.XB = maxps;
   const size_t kcap = pad2(maxps);
-  const size_t smem = sizeof(float2) * (2 * kcap + (size_t)NG * P::LS + pad2(A.X)) +
-                      (1 + P::STARTS) * kcap * (P::TABULATE ? sizeof(float2) : sizeof(short));
+  const size_t smem = sizeof(float2) * (P::NK * kcap + (size_t)NG * P::LS + pad2(A.X)) +
+                      P::TABLES * kcap * (P::TABULATE ? sizeof(float2) : sizeof(short));
   ME_TRY(check_cuda(allow_smem(fast_adj_kernel<Y>, smem), "adj smem"));
   dim3 grid(nb, (A.X + NG - 1) / NG, A.Z);
   count_launch();
