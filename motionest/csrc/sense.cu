@@ -32,8 +32,14 @@ namespace me {
     if (_rc != ME_OK) return _rc; \
   } while (0)
 
-// Resident CTAs per SM that the compile-time SENSE kernels are built for.
-__host__ __device__ constexpr int sense_min_ctas(int y) { return line_threads(y) == 8 ? 3 : 2; }
+// Resident CTAs per SM that the compile-time forward is built for.  Lines of eight threads leave room
+// for three unless a thread holds eight samples, whose accumulators and indices then spill (24 to
+// 112 points, 32 planes, 8 coils, 8 shots of 1,500 samples, 80 and 128 registers: 143 and 130 us at
+// 24, 165 and 150 at 56, 227 and 196 at 112; 128 points 202 and 206).  Four samples a thread hold
+// three (1,000 samples at 56 and 112 points, three and two CTAs: 111 and 119 us, 156 and 158).
+__host__ __device__ constexpr int sense_min_ctas(int y, int mpt) {
+  return line_threads(y) == 8 && mpt <= 4 ? 3 : 2;
+}
 
 // Gauss-Newton sums of one sample: |r|^2, Re(conj(r) J_p) and Re(conj(J_p) J_q) for q >= p.
 __device__ __forceinline__ void lm_accumulate(double (&st)[kLmStats], float2 r, const float2 (&J)[6]) {
@@ -313,7 +319,7 @@ struct SampleSteps {
 };
 
 template <int Y, int MPT, int MODE>
-__global__ void __launch_bounds__(kThreads, sense_min_ctas(Y)) fast_fwd_kernel(const FwdArgs A) {
+__global__ void __launch_bounds__(kThreads, sense_min_ctas(Y, MPT)) fast_fwd_kernel(const FwdArgs A) {
   static_assert(MODE == FWD_K || MODE == FWD_RESID, "one volume per CTA");
   using P = FwdPlan<Y>;
   using F = typename P::F;
