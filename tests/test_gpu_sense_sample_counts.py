@@ -49,11 +49,15 @@ def test_forward_sample_counts(Y, n):
     assert (err / ref2) ** 0.5 < (2.0e-7 if n > 1 else 6.0e-7)
 
 
-@pytest.mark.parametrize("Y", [48, 56, 96, 112])
-def test_forward_time_grows_slower_than_samples(Y):
+@pytest.mark.parametrize("Y, few, many, limit", [(48, 1000, 1500, 1.42), (56, 1000, 1500, 1.42),
+                                                 (96, 1000, 1500, 1.42), (112, 1000, 1500, 1.42),
+                                                 (224, 400, 2000, 2.0)])
+def test_forward_time_grows_slower_than_samples(Y, few, many, limit):
     """1,500 samples a shot take less than 1.42 times the time of 1,000: half as many again, less the
     share of the FFTs (a sixth at least), which do not grow.  With eight samples a thread in 80
-    registers the kernel spilled and took 1.46 to 1.51 times."""
+    registers the kernel spilled and took 1.46 to 1.51 times.  At 224 points the FFTs are two
+    thirds at 400 samples, so that five times as many take less than twice the time; with the steps
+    read out of the twiddle table in every chunk they took 2.07 times."""
     def median_us(n):
         _, _, _, call = _forward(128, Y, 32, 8, 8, n, 7)
         for _ in range(3):
@@ -70,4 +74,4 @@ def test_forward_time_grows_slower_than_samples(Y):
             t.append(a.elapsed_time(b))
         return sorted(t)[4]
 
-    assert median_us(1500) < 1.42 * median_us(1000)
+    assert median_us(many) < limit * median_us(few)
