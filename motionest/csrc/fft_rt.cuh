@@ -4,8 +4,9 @@
 // most up to 512.
 //
 // A stage is one register DFT per work item, its radix picked by a switch that the whole CTA
-// takes the same way, so the DFTs stay unrolled and in registers while a kernel serves every
-// length.  Items are dealt to threads over all of a tile's lines (thread i has the one item i
+// takes the same way, so the DFTs stay unrolled while a kernel serves every length.  A kernel's
+// registers are those of its largest radix: R2 above 16 has kernels of its own, of 128 registers;
+// the stack frames are 80 bytes at most there and 48 bytes elsewhere.  Items are dealt to threads over all of a tile's lines (thread i has the one item i
 // of a stage), so a radix that is no power of two leaves whole warps idle at the end of the
 // CTA rather than lanes in every warp:
 //   stage 1: item (line b, j < R2) transforms x[j + r R2], r < R1, into row j of the line's
@@ -24,7 +25,7 @@ namespace me {
 #define ME_RT_SMALL(X) \
   X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
 #define ME_RT_LARGE(X) \
-  ME_RT_SMALL(X) X(18) X(20) X(21) X(22) X(24) X(25) X(26) X(27) X(28) X(30) X(32)
+  X(18) X(20) X(21) X(22) X(24) X(25) X(26) X(27) X(28) X(30) X(32)
 
 constexpr int kRtMaxR1 = 16;
 
@@ -89,6 +90,19 @@ __device__ __forceinline__ void rt_init_twiddles(float2* tw, const RtPlan& P) {
     sincospi(-2.0 * (double)(r * k) / (double)P.n, &s, &c);
     tw[i] = make_float2((float)c, (float)s);
   }
+}
+
+// v, hidden from the compiler's knowledge of how it came about.  The multiples r * step of a stride
+// that does not change between tiles would otherwise be kept in registers across the tile loop, a
+// set for every radix of the switches, and spilled: the line passes had stack frames of 0.5 to
+// 4.9 KB, which also size the local memory that the device sets aside for all threads.
+__device__ __forceinline__ int fresh(int v) {
+  asm volatile("" : "+r"(v));
+  return v;
+}
+__device__ __forceinline__ i64 fresh(i64 v) {
+  asm volatile("" : "+l"(v));
+  return v;
 }
 
 // Calls f(std::integral_constant<int, R>) with the radix of a stage.

@@ -5,12 +5,16 @@
 // The first stage reads its elements straight from global memory into registers and the last
 // one writes them straight back, coalesced over the lines of the tile where the pass axis is
 // strided and along the line where it is contiguous, so a line crosses shared memory twice in
-// each direction instead of four times and no alignment is asked of the volume.  What bounds it
-// is the latency of those loads: three CTAs per SM (two for R2 > 16) cover it.  Measured: one
-// partial derivative of a 180x150x126 image (12 passes, three of them dual) 3.13 ms on the
-// Stockham engine of line_pass_kernel, 0.70 ms here; ten passes over 20 volumes of 160x150x126
-// 34 -> 4.3 ms.  Not used where a compile-time plan exists: at 256x224x176, 64 volumes, ten
-// passes take 37.0 ms here and 26.1 ms on the TMA tiles of tma_pass_kernel.
+// each direction instead of four times and no alignment is asked of the volume.  What bounds it:
+// the latency of those loads, which three CTAs per SM (two for R2 > 16 and the dual modes) cover,
+// and instruction issue.  Strides are taken through `fresh` (fft_rt.cuh) and the dual modes hold one
+// spectrum at a time, so that next to nothing is spilled; with all their multiples kept and both
+// spectra held, one partial derivative (12 passes, three of them dual) of a 27x125x216 image took
+// 1,146 us instead of 234 (on the Stockham engine of line_pass_kernel 911), of 60x63x50 210 instead
+// of 113, of 180x150x126 682 instead of 456 (Stockham 3,154), and the device set 1.2 GB aside for
+// local memory.  Not used where a compile-time plan exists: at 256x224x176, 64 volumes, ten
+// passes took 37.0 ms here and 26.1 ms on the TMA tiles of tma_pass_kernel (both measured before
+// the spills were gone).
 #pragma once
 #include <algorithm>
 #include <atomic>
@@ -121,7 +125,8 @@ __global__ void __launch_bounds__(256, (LARGE || MODE == PM_DUAL_IN || MODE == P
     if (MODE != PM_INV && has1) {
       int u, v;
       const i64 base = line(b1, u, v) + (i64)j1 * sa;
-      const i64 step = (i64)R2 * sa;
+      const i64 step = fresh((i64)R2 * sa);
+      const int sk = fresh(ix.sk);
       const bool live = b1 < nl;
       rt_switch1(R1, [&](auto rc) {
         constexpr int R = decltype(rc)::value;
@@ -130,11 +135,11 @@ __global__ void __launch_bounds__(256, (LARGE || MODE == PM_DUAL_IN || MODE == P
           const float2* src = (q == 0 ? A.in0 : A.in1) + (i64)vol * A.in_vs + base;
           float2 x[R];
 #pragma unroll
-          for (int r = 0; r < R; r++) x[r] = live ? src[r * step] : make_float2(0.f, 0.f);
+          for (int r = 0; r < R; r++, src += step) x[r] = live ? *src : make_float2(0.f, 0.f);
           RDft<R, false>::run(x);
           float2* dst = (q == 0 ? reg0 : reg1) + ix.at(b1, j1, 0);
 #pragma unroll
-          for (int r = 0; r < R; r++) dst[r * ix.sk] = x[r];
+          for (int r = 0; r < R; r++, dst += sk) *dst = x[r];
         }
       });
     }
@@ -158,7 +163,7 @@ __global__ void __launch_bounds__(256, (LARGE || MODE == PM_DUAL_IN || MODE == P
     if (has2) {
       int u, v;
       const i64 base = line(b2, u, v) + (i64)k2 * sa;
-      const i64 step = (i64)R1 * sa;
+      const i64 step = fresh((i64)R1 * sa);
       const bool live = b2 < nl;
       int c[3];
       c[A.au] = u;
@@ -188,18 +193,18 @@ __global__ void __launch_bounds__(256, (LARGE || MODE == PM_DUAL_IN || MODE == P
       rt_switch2<LARGE>(R2, [&](auto rc) {
         constexpr int R = decltype(rc)::value;
         auto forward = [&](const float2* col, float2 (&X)[R]) {
+          const int sj = fresh(ix.sj), st = fresh(R1);
+          const float2* w = tw + k2;
 #pragma unroll
-          for (int r = 0; r < R; r++) {
-            const float2 y = col[r * ix.sj];
-            X[r] = (r == 0) ? y : cmul(y, tw[r * R1 + k2]);
-          }
+          for (int r = 0; r < R; r++, col += sj, w += st) X[r] = (r == 0) ? *col : cmul(*col, *w);
           RDft<R, false>::run(X);
         };
         auto inverse = [&](float2* col, float2 (&X)[R]) {
           RDft<R, true>::run(X);
+          const int sj = fresh(ix.sj), st = fresh(R1);
+          const float2* w = tw + k2;
 #pragma unroll
-          for (int r = 0; r < R; r++)
-            col[r * ix.sj] = (r == 0) ? X[r] : cmulc(X[r], tw[r * R1 + k2]);
+          for (int r = 0; r < R; r++, col += sj, w += st) *col = (r == 0) ? X[r] : cmulc(X[r], *w);
         };
         // X[r] (index k + r R1) times the factors of phase q: the line's table entry times the
         // thread's own, one rounding each
@@ -215,9 +220,10 @@ __global__ void __launch_bounds__(256, (LARGE || MODE == PM_DUAL_IN || MODE == P
               const double r_o = ph.rvec ? ph.rvec[o] : 0.0;
               const float dmr = (float)(coef_s[q].dm * r_o * (kTwoPi / N));
               const float tdr = (float)(kTwoPi / N);
+              int n = fresh(k2);
+              const int dn = fresh(R1);
 #pragma unroll
-              for (int r = 0; r < R; r++) {
-                const int n = k2 + r * R1;
+              for (int r = 0; r < R; r++, n += dn) {
                 const float mm = (float)(n - (n >= half ? N : 0)) + (float)odd_h;
                 float2 f = cmul(e[q], st[(r == rsel ? R2 : r) * B]);
                 if (ph.deriv) f = cscale(ph.conj ? mul_mi(f) : mul_i(f), dmr * mm);
@@ -231,40 +237,52 @@ __global__ void __launch_bounds__(256, (LARGE || MODE == PM_DUAL_IN || MODE == P
             }
           } else {
             general(q, col);
+            const int sj = fresh(ix.sj);
 #pragma unroll
-            for (int r = 0; r < R; r++) X[r] = cmul(X[r], col[r * ix.sj]);
+            for (int r = 0; r < R; r++, col += sj) X[r] = cmul(X[r], *col);
           }
         };
         float2 X[R];
         if (MODE == PM_INV) {
           const float2* src = A.in0 + (i64)vol * A.in_vs + base;
 #pragma unroll
-          for (int r = 0; r < R; r++) X[r] = live ? src[r * step] : make_float2(0.f, 0.f);
+          for (int r = 0; r < R; r++, src += step) X[r] = live ? *src : make_float2(0.f, 0.f);
         } else {
           forward(col0, X);
         }
-        if (MODE == PM_DUAL_IN) {
-          float2 Y[R];
-          factor(0, col0, X);
-          forward(col1, Y);
-          factor(1, col1, Y);
+        // The dual modes park a spectrum in a column that this thread alone reads and writes, so
+        // that one of them is in registers at a time.
+        auto park = [&](float2* col) {
+          const int sj = fresh(ix.sj);
 #pragma unroll
-          for (int r = 0; r < R; r++) X[r] = cadd(X[r], Y[r]);
+          for (int r = 0; r < R; r++, col += sj) *col = X[r];
+        };
+        if (MODE == PM_DUAL_IN) {
+          factor(0, col0, X);
+          park(col0);
+          forward(col1, X);
+          factor(1, col1, X);
+          const float2* first = col0;
+          const int sj = fresh(ix.sj);
+#pragma unroll
+          for (int r = 0; r < R; r++, first += sj) X[r] = cadd(*first, X[r]);
           inverse(col0, X);
         } else if (MODE == PM_DUAL_OUT) {
-          float2 Y[R];
-#pragma unroll
-          for (int r = 0; r < R; r++) Y[r] = X[r];
+          park(col1);
           factor(0, col0, X);
           inverse(col0, X);
-          factor(1, col1, Y);
-          inverse(col1, Y);
+          const float2* parked = col1;
+          const int sj = fresh(ix.sj);
+#pragma unroll
+          for (int r = 0; r < R; r++, parked += sj) X[r] = *parked;
+          factor(1, col1, X);
+          inverse(col1, X);
         } else if (MODE == PM_FWD) {
           factor(0, col0, X);
           if (live) {
             float2* dst = A.out0 + (i64)vol * A.out_vs + base;
 #pragma unroll
-            for (int r = 0; r < R; r++) dst[r * step] = X[r];
+            for (int r = 0; r < R; r++, dst += step) *dst = X[r];
           }
         } else {
           factor(0, col0, X);
@@ -279,7 +297,8 @@ __global__ void __launch_bounds__(256, (LARGE || MODE == PM_DUAL_IN || MODE == P
       // tile's first stage, so no barrier separates the two
       int u, v;
       const i64 base = line(b1, u, v) + (i64)j1 * sa;
-      const i64 step = (i64)R2 * sa;
+      const i64 step = fresh((i64)R2 * sa);
+      const int sk = fresh(ix.sk);
       rt_switch1(R1, [&](auto rc) {
         constexpr int R = decltype(rc)::value;
 #pragma unroll
@@ -287,15 +306,15 @@ __global__ void __launch_bounds__(256, (LARGE || MODE == PM_DUAL_IN || MODE == P
           const float2* src = (q == 0 ? reg0 : reg1) + ix.at(b1, j1, 0);
           float2 x[R];
 #pragma unroll
-          for (int r = 0; r < R; r++) x[r] = src[r * ix.sk];
+          for (int r = 0; r < R; r++, src += sk) x[r] = *src;
           RDft<R, true>::run(x);
           float2* dst = (q == 0 ? A.out0 : A.out1) + (i64)vol * A.out_vs + base;
           if (q == 0 && A.accum) {
 #pragma unroll
-            for (int r = 0; r < R; r++) dst[r * step] = cadd(x[r], dst[r * step]);
+            for (int r = 0; r < R; r++, dst += step) *dst = cadd(x[r], *dst);
           } else {
 #pragma unroll
-            for (int r = 0; r < R; r++) dst[r * step] = x[r];
+            for (int r = 0; r < R; r++, dst += step) *dst = x[r];
           }
         }
       });

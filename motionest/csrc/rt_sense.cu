@@ -247,14 +247,16 @@ __global__ void __launch_bounds__(kThreads, 2)
     if (has2) {
       rt_switch2<LARGE>(R2, [&](auto rc) {
         constexpr int R = decltype(rc)::value;
-        const float2* src = H + g2 * T.ys + k2;
+        const float2 *src = H + g2 * T.ys + k2, *w2 = tw + k2;
+        const int step = fresh(R1), row = fresh(S1);
         float2 v[R];
 #pragma unroll
-        for (int r = 0; r < R; r++) v[r] = src[r * R1];
+        for (int r = 0; r < R; r++, src += step) v[r] = *src;
         RDft<R, true>::run(v);
         float2* dst = tab + g2 * T.ls + k2;
 #pragma unroll
-        for (int r = 0; r < R; r++) dst[r * S1] = (r == 0) ? v[0] : cmulc(v[r], tw[r * R1 + k2]);
+        for (int r = 0; r < R; r++, dst += row, w2 += step)
+          *dst = (r == 0) ? v[0] : cmulc(v[r], *w2);
       });
     }
     __syncthreads();
