@@ -120,14 +120,20 @@ class SenseProblem:
             tune(self)
 
     def _default_lm_batch(self):
-        """Shots per launch of the motion step: as many as 1.5 GB of workspace hold, at least 8.
+        """Shots per launch of the motion step: as many as 1.5 GB of workspace hold, at least 8.  More
+        than 256 MB above eight shots' worth are taken up to a 32nd of the device's free memory
+        only (a process with many problems); asking for that takes 70 us.
 
-        A pass over eight volumes of 64x64x48 is over before its launch is paid for (16 shots in
-        one batch instead of two: 2.18 -> 1.70 ms); from 128x112x88 on the passes fill the GPU
-        with eight, and at full size more shots only cost memory."""
+        A pass over eight volumes of 64x64x48 is over before its launch is paid for (8 coils, 64
+        shots in batches of 8, 16, 32 and 64: 7.1, 6.0, 5.4 and 5.2 ms); from 128x112x88 on the
+        passes fill the GPU with eight (32.4, 30.8, 29.9 and 29.5 ms), and at full size more shots
+        only cost memory."""
         lib = _lib.load()
-        one = lib.me_lm_workspace_bytes(self.ref, 1)
-        return max(8, min(self.nshots, int(1.5e9 // max(one, 1))))
+        one = max(lib.me_lm_workspace_bytes(self.ref, 1), 1)
+        most = max(8, min(self.nshots, int(1.5e9 // one)))
+        if (most - 8) * one <= 256 << 20:
+            return most
+        return max(8, min(most, int(torch.cuda.mem_get_info(self.device)[0] / 32 // one)))
 
     def set_batches(self, batch, lm_batch):
         """Shots per launch for the SENSE operators and for the LM statistics; grows the

@@ -132,7 +132,8 @@ def generate_corrupted_kspace(gt_img, mps, A, transforms):
     t = torch.as_tensor(np.asarray(transforms if not isinstance(transforms, torch.Tensor)
                                    else transforms.cpu(), dtype=np.float64)).cuda()
     kgrid, rkgrid = compute_transform_grids_voxel(tuple(gt.shape), [1, 1, 1])
-    pb = SenseProblem(None, mps_u, planes, kgrid, rkgrid, t)
+    # (forward only: no motion step, so no workspace for its batches)
+    pb = SenseProblem(None, mps_u, planes, kgrid, rkgrid, t, lm_batch=1)
     K = pb.forward(xyz_to_zxy(gt), t)
     C = mps_u.shape[0]
     ksp_h = torch.zeros((C,) + tuple(gt.shape), dtype=torch.complex64, device=gt.device)
