@@ -58,7 +58,10 @@ extern "C" int me_sample_lists(const unsigned char* planes, int nshots, int nx, 
                                int* ky_order) {
   if (!planes || !shot_off || !ky_off || !ky_order || (total > 0 && (!kx || !ky)))
     return fail("me_sample_lists: NULL pointer");
-  if (nshots < 1 || nx < 1 || ny < 1 || (i64)nx * ny > 0x7fffffff) return fail("me_sample_lists: dims must be positive");
+  if (nshots < 1 || nx < 1 || ny < 1 || (i64)nx * ny > 0x7fffffff)
+    return fail("me_sample_lists: dims must be positive, nx * ny below 2^31");
+  if (total < 0 || total > 0x7fffffff)  // the offsets are 32-bit
+    return fail("me_sample_lists: `total` outside 0 .. 2^31 - 1");
   try {
     std::vector<int> at(ny), sorted, next, found;
     const int split = (ny > 128 && ny < 256) ? 256 - ny : 0;

@@ -128,9 +128,9 @@ def _native_lists(planes):
         return None
     S, X, Y = planes.shape
     total = int(np.count_nonzero(planes))
-    out = [np.empty(n, np.int32) for n in (S + 1, total, total, S * (Y + 1), S * Y)]
-    if S == 0 or X == 0 or Y == 0 or total > np.iinfo(np.int32).max:
+    if 0 in (S, X, Y) or max(total, X * Y) > np.iinfo(np.int32).max:
         return None
+    out = [np.empty(n, np.int32) for n in (S + 1, total, total, S * (Y + 1), S * Y)]
     _lib.check(lib.me_sample_lists(planes.ctypes.data, S, X, Y, total,
                                    *(a.ctypes.data for a in out)))
     return out

@@ -140,3 +140,17 @@ def test_native_lists_match_python(S, X, Y, share):
     for a, b in zip(got, want):
         assert a.dtype == np.int32
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("total", [-1, 2**31, 2**40])
+def test_native_lists_refuse_totals_beyond_their_offsets(total):
+    """The offsets are 32-bit: a total that they cannot hold is refused by name, before anything is
+    written."""
+    from motionest import _lib
+    lib = _lib.load()
+    planes = np.ones((1, 2, 3), np.uint8)
+    out = [np.full(n, -7, np.int32) for n in (2, 6, 6, 4, 3)]
+    rc = lib.me_sample_lists(planes.ctypes.data, 1, 2, 3, total, *(a.ctypes.data for a in out))
+    assert rc != 0
+    assert "2^31 - 1" in lib.me_last_error().decode()
+    assert all((a == -7).all() for a in out)
