@@ -18,6 +18,10 @@
 
 namespace me {
 
+// Planes of a launch: more (only calls on caller-transformed volumes can have them, whose z axis
+// is no line) go to the kernels of sense.cu, which count them along x.
+constexpr int kMaxGridZ = 65535;
+
 constexpr int kOctet = 8;  // rows per H-building item; NR is a multiple
 
 // Rows per CTA for a plan.
@@ -319,7 +323,8 @@ static int launch_rt_fwd_m(FwdArgs& A, const RtSense& T, int maxps, int nb, cuda
 
 int try_rt_fwd(FwdArgs& A, int mode, int maxps, int nb, cudaStream_t st) {
   RtSense T;
-  if ((mode != FWD_K && mode != FWD_RESID) || !rt_sense_plan(A.Y, &T)) return -1;
+  if ((mode != FWD_K && mode != FWD_RESID) || A.Z > kMaxGridZ || !rt_sense_plan(A.Y, &T))
+    return -1;
   // several coils per CTA while that leaves some ten waves of CTAs
   const i64 ctas = (i64)nb * A.vps * A.C * A.Z;
   T.cg = (int)std::max<i64>(1, std::min<i64>(std::min(A.C, 8), ctas / (148 * 3 * 10)));
@@ -344,7 +349,7 @@ static int launch_rt_adj(AdjArgs& A, const RtSense& T, int nb, cudaStream_t st) 
 
 int try_rt_adj(AdjArgs& A, int maxps, int nb, cudaStream_t st) {
   RtSense T;
-  if (!rt_sense_plan(A.Y, &T)) return -1;
+  if (A.Z > kMaxGridZ || !rt_sense_plan(A.Y, &T)) return -1;
   A.XB = (maxps + 1) & ~1;
   return T.P.large() ? launch_rt_adj<true>(A, T, nb, st) : launch_rt_adj<false>(A, T, nb, st);
 }
