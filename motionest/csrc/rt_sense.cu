@@ -326,8 +326,11 @@ int try_rt_fwd(FwdArgs& A, int mode, int maxps, int nb, cudaStream_t st) {
   if ((mode != FWD_K && mode != FWD_RESID) || A.Z > kMaxGridZ || !rt_sense_plan(A.Y, &T))
     return -1;
   // several coils per CTA while that leaves some ten waves of CTAs
-  const i64 ctas = (i64)nb * A.vps * A.C * A.Z;
-  T.cg = (int)std::max<i64>(1, std::min<i64>(std::min(A.C, 8), ctas / (148 * 3 * 10)));
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const i64 ctas = (i64)nb * A.vps * A.C * A.Z, wave = 3LL * std::max(1, sms);
+  T.cg = (int)std::max<i64>(1, std::min<i64>(std::min(A.C, 8), ctas / (10 * wave)));
   if (mode == FWD_K)
     return T.P.large() ? launch_rt_fwd_m<FWD_K, true>(A, T, maxps, nb, st)
                        : launch_rt_fwd_m<FWD_K, false>(A, T, maxps, nb, st);
