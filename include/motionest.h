@@ -100,12 +100,12 @@ long long me_launch_count(void);
  * counterpart in the reference (CuPy and cuFFT have no such waits).
  * me_wait_status synchronises the current device, returns the OR of the recorded bits in
  * *status (0: no wait ran out; 4 line pass, 0x100 the self-test; 1 and 2, the SENSE kernels, no
- * longer occur: these stage nothing) and clears them.  Results of launches before a non-zero status are not to be
- * trusted.  me_wait_selftest launches one CTA whose barrier never completes (one arrival short
+ * longer occur: these stage nothing) and clears them.  Results of launches before a non-zero
+ * status are not to be trusted.  me_wait_selftest launches one CTA whose barrier never completes (one arrival short
  * of its count) and whose wait gives up after limit_cycles (1 .. 2^31) clock cycles; the next
  * me_wait_status then reports 0x100. */
-#define ME_WAIT_SENSE_FWD 0x1u
-#define ME_WAIT_SENSE_ADJ 0x2u
+#define ME_WAIT_SENSE_FWD 0x1u /* kept for programs that name it; never set */
+#define ME_WAIT_SENSE_ADJ 0x2u /* the same */
 #define ME_WAIT_LINE_PASS 0x4u
 #define ME_WAIT_SELFTEST 0x100u
 int me_wait_status(unsigned* status);

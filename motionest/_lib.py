@@ -142,7 +142,7 @@ _SIGS = {
     "me_wait_selftest": (ctypes.c_int, [c_i64, c_ptr]),
 }
 
-# me_wait_status bits
+# me_wait_status bits (those of the SENSE kernels are never set: these wait for nothing)
 ME_WAIT_SENSE_FWD = 0x1
 ME_WAIT_SENSE_ADJ = 0x2
 ME_WAIT_LINE_PASS = 0x4

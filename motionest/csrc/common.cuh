@@ -89,12 +89,7 @@ __device__ __forceinline__ float2 cscale2(float2 a, float hi, float lo) {
   return make_float2(fmaf(a.x, hi, a.x * lo), fmaf(a.y, hi, a.y * lo));
 }
 
-// Ampere-style asynchronous global -> shared copies (16 bytes; both addresses 16-byte aligned).
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem_src) : "memory");
-}
-// 8-byte variant (both addresses 8-byte aligned), cached in L1.
+// Asynchronous global -> shared copy of 8 bytes (both addresses 8-byte aligned), cached in L1.
 __device__ __forceinline__ void cp_async8(void* smem_dst, const void* gmem_src) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem_src) : "memory");
