@@ -494,8 +494,11 @@ static bool tma_pass_setup(int mode, const PassArgs& A, bool* strided, PassTma* 
   if (other % 2 != 0 || A.st[A.au] % 2 != 0) return false;
   const i64 lim = (i64)1 << 36;  // strides below 2^40 bytes
   if (other >= lim || A.st[A.au] >= lim || A.in_vs >= lim || A.out_vs >= lim) return false;
-  // tiles of fewer than eight lines in use are better packed by the cp.async kernel
-  if (s && A.dims[A.av] % kTileLines != 0 && A.dims[A.av] < 2 * kTileLines) return false;
+  // A row's last tile may hold a few lines only and the tensor copy is still the better one (ten passes
+  // of 128 x Y x 96, cp.async and TMA: Y = 18 89 and 68 us, 24 97 and 76, 30 95 and 73; 16
+  // volumes, Y = 18 349 and 337 us, 24 466 and 403, 30 488 and 371).  Rows shorter than a tile
+  // would be padding in every tile.
+  if (s && A.dims[A.av] < kTileLines) return false;
   const int nin = (mode == PM_DUAL_IN) ? 2 : 1, nout = (mode == PM_DUAL_OUT) ? 2 : 1;
   const float2* ins[2] = {A.in0, A.in1};
   float2* outs[2] = {A.out0, A.out1};
