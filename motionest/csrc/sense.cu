@@ -701,12 +701,12 @@ __global__ void __launch_bounds__(kThreads, Y <= 64 ? 3 : 2) fast_adj_kernel(con
     __syncthreads();
     if (P::NK == 1 && c + 1 < A.C) issue(c + 1);
     // Added to the sum over the coils as one term, the product rounds it once; fused into it, twice
-    // (128 points, 32 coils: 1.6e-7 from 64 bits and, fused, 2.1e-7).  Sixteen threads a line keep
-    // the fused form: the other one spills at 192 and 224 points (1.5 to 5% there).
+    // (128 points, 32 coils: 1.6e-7 from 64 bits and, fused, 2.1e-7).  144 to 224 points keep the
+    // fused form: the other one spills at 192 and 224 (1.5 to 5% there).
     F::inverse(slots, j, [&](int q, int, float2 v) {
       if (!live) return;
       const float2 m = __ldg(ms + q * G);
-      w[q] = G == 8 ? cadd(w[q], cmulc(v, m)) : cfmac(v, m, w[q]);
+      w[q] = NSPLIT == 0 ? cadd(w[q], cmulc(v, m)) : cfmac(v, m, w[q]);
     });
   }
   if (live) {

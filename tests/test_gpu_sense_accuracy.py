@@ -62,7 +62,7 @@ def test_forward_against_fp64(X, Y):
     assert _rel(K.reshape(ref.shape).to(torch.complex128), ref) < 2.0e-7
 
 
-@pytest.mark.parametrize("Y", [48, 64, 72, 88, 96, 112, 128, 40, 80, 90, 150, 160, 200])
+@pytest.mark.parametrize("Y", [48, 64, 72, 88, 96, 112, 128, 256, 40, 80, 90, 150, 160, 200])
 @pytest.mark.parametrize("X", [128, 150])
 def test_adjoint_against_fp64(X, Y):
     """Relative L2 below 1.75e-7 with 32 coils.  One rounding a coil (2.5e-8 of the running sum, which
