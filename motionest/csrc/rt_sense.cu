@@ -127,8 +127,8 @@ __global__ void __launch_bounds__(kThreads, (MPT > 4 || LARGE) ? 2 : 3)
       }
       __syncthreads();
       // sample sums over the chunk's rows by Horner's rule in four chains, each stepping by W^4kx
-      // (rows past X hold zeros): a chain of 31 rows would carry the rounding of its step up to
-      // the 15th power
+      // (rows past X hold zeros): of 32 rows, a chain carries the rounding of its step up to the
+      // 7th power; two chains would to the 15th
 #pragma unroll
       for (int m = 0; m < MPT; m++) {
         const int jj = tid + m * kThreads;

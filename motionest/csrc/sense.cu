@@ -254,7 +254,7 @@ __device__ __forceinline__ void init_twiddles_any(float2* tw, int n) {
 // shared-memory traffic than it hid: without it, and with the plans of LineFft, the forward went
 // from 55.8 to 53.5 ms and the adjoint from 63.6 to 60.8 ms at 256x224x176, 32 coils, 64 shots,
 // and from 2.50 to 1.68 and 3.47 to 2.10 ms at 128x112x88, 16 coils, 32 shots (three CTAs per SM
-// instead of two for the forward up to 128 points).  What bounds both: instruction issue and the
+// instead of two for the forward up to 128 points and four samples a thread).  What bounds both: instruction issue and the
 // shared-memory pipe together (transposes, columns of the sample sums, H rows).
 
 // This thread's row group g and its place j < G in it: sixteen threads of one row to a half warp,
@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(kThreads, sense_min_ctas(Y, MPT)) fast_fwd_ker
 
 // Gauss-Newton statistics of the LM step straight from the seven volumes of each shot (T x and
 // its six partials, [shot][7] in A.vols): the forward model of all seven runs in one CTA per
-// (shot, coil, plane), each chunk's map rows staged once for the seven volumes, and the sampled
+// (shot, coil, plane), each chunk's map rows read seven times in turn (from L1), and the sampled
 // values J_v = M_s F C U_v are contracted in registers into e0 = |J_0 - y|^2, g_p = Re<J_0 - y,
 // J_p> and H_pq = Re<J_p, J_q> (transform_estimation.py:39-68) instead of being written out.
 // The sums per sample and their block reduction are those of lm_stats_kernel, in the same order,
